@@ -97,3 +97,25 @@ def test_device_entry_matches_host_entry():
 def test_odd_extents_are_rejected():
     with pytest.raises(update.UpdateError):
         update.heatbath(update.unit_config((4, 4, 4, 5)), (4, 4, 4, 5), 6.0, 1)
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 4, 2, 2), (10, 6, 4, 6), (8, 8, 8, 16)])
+def test_links_outside_su3_keep_all_columns(dims):
+    """Links times a common phase are no longer the cross product of their
+    first two columns and are kept whole; U S^dag is unchanged by the phase,
+    so the over-relaxed links are those of the SU(3) links times the phase."""
+    V = int(np.prod(dims))
+    rng = np.random.default_rng(5)
+    z = 8 * np.eye(3)[:, :2] + rng.normal(size=(V, 4, 3, 2)) + 1j * rng.normal(size=(V, 4, 3, 2))
+    c0 = z[..., 0] / np.linalg.norm(z[..., 0], axis=-1, keepdims=True)
+    c1 = z[..., 1] - np.sum(np.conj(c0) * z[..., 1], axis=-1, keepdims=True) * c0
+    c1 /= np.linalg.norm(c1, axis=-1, keepdims=True)
+    U = np.stack([c0, c1, np.conj(np.cross(c0, c1))], axis=-1)
+    ph = np.exp(0.3j)
+    a = update.overrelax(U, dims, 2)
+    b = update.overrelax(ph * U, dims, 2)
+    # two sweeps of products and rotations, rounding at 1e-16 each over the
+    # size of the subgroups they normalise (links with a common mean keep
+    # those of order one; on independent links some are near zero)
+    assert np.abs(b - ph * a).max() < 1e-12
+    assert np.abs(np.linalg.det(a) - 1).max() < 1e-12
