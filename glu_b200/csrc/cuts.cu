@@ -17,6 +17,9 @@
 //                 writes the packed fields first
 //   k_cut_zt      z and t transforms of tiles of x columns
 //                 (both also as k_cut_*_ct with compile-time extents)
+//   k_cut_pxy, k_cut_pz, k_cut_pt  instead of the full transforms, where the
+//                 cut keeps few momenta of each axis: every axis is summed
+//                 into its kept components alone
 //   k_cut_gather  per listed momentum: A_mu(p) for all 9 colour entries
 //                 from the packed transforms at p and -p (the transform of
 //                 a real field R obeys R(-p) = conj R(p), and of conj(f)
@@ -359,6 +362,153 @@ __global__ void __launch_bounds__(128) k_cut_log_pack(CutCtx c) {
   for (int q = 0; q < 4; q++) c.F[(size_t)(mu * 4 + q) * c.V + site] = q4[q];
 }
 
+// ---------------------------------------------------------------------
+// Partial transforms: a cut keeps the momenta |n_mu| <= b_mu of each axis (5
+// of 32 with MAXMOM 4, 9 with 20), so each axis is summed directly into its
+// K_mu = 2 b_mu + 1 components (all L_mu where that is fewer): x and y while
+// the links are read, which leaves K_x K_y / (L_x L_y) of the fields, then z
+// and t.  Component n sits at n, -n at K - n.  The sums of n and -n share
+// their four products with cos and sin.  32^3 x 64, MAXMOM 4: x and y
+// 0.509 -> 0.251 ms, z and t 0.412 -> 0.028 ms, 0.185 ms of it the links at the
+// copy bandwidth; MAXMOM 20 with logarithms, which bound it, 0.862 + 0.412 ->
+// 0.820 + 0.038 ms.
+// The fields of a direction are stored in the order (q + mu) & 3, which
+// spreads the four directions' stores over the banks.
+struct PartCtx {
+  int L[4], b[4], K[4];
+  const C2 *links;
+  C2 *F1, *F2, *F3;  // [t z][C], [t][Kz][C], [Kt][Kz][C], C = Ky Kx 16
+  const C2 *tw;
+  int tw_off[4];
+};
+
+constexpr int kPartThreads = 256;
+constexpr int kPartSites = 128;   // sites of a chunk of rows, at least
+constexpr int kPartTasks = 8;     // y sums a thread holds, at most
+
+// rows of x in one chunk
+__host__ __device__ __forceinline__ int part_rows(int lx, int ly) {
+  const int r = (kPartSites + lx - 1) / lx;
+  return r < ly ? r : ly;
+}
+__host__ __device__ __forceinline__ size_t part_smem(int lx, int ly, int kx) {
+  return (size_t)(part_rows(lx, ly) * (lx + kx) * kNF + lx + ly) * sizeof(C2);
+}
+
+// v += f (cos, sin) of the pair of components n and -n: p = sum f cos,
+// q = sum f sin
+__device__ __forceinline__ void pair_add(C2 f, C2 w, C2 *p, C2 *q) {
+  p->x = fma(f.x, w.x, p->x);
+  p->y = fma(f.y, w.x, p->y);
+  q->x = fma(f.x, -w.y, q->x);
+  q->y = fma(f.y, -w.y, q->y);
+}
+// sum f e^{+i n theta} and sum f e^{-i n theta}
+__device__ __forceinline__ C2 pair_pos(C2 p, C2 q) { return mk<double>(p.x - q.y, p.y + q.x); }
+__device__ __forceinline__ C2 pair_neg(C2 p, C2 q) { return mk<double>(p.x + q.y, p.y - q.x); }
+
+// Lie fields of one xy plane and their kept x and y components; NT: y sums
+// per thread
+template <bool LOG, int NT>
+__global__ void __launch_bounds__(kPartThreads) k_cut_pxy(PartCtx c) {
+  extern __shared__ unsigned char smem_raw[];
+  const int Lx = c.L[0], Ly = c.L[1], Kx = c.K[0], Ky = c.K[1], R = part_rows(Lx, Ly);
+  C2 *A = reinterpret_cast<C2 *>(smem_raw);  // [R][Lx][16]
+  C2 *X = A + (size_t)R * Lx * kNF;          // [R][Kx][16]
+  C2 *twx = X + (size_t)R * Kx * kNF;
+  C2 *twy = twx + Lx;
+  for (int k = threadIdx.x; k < Lx; k += kPartThreads) twx[k] = c.tw[c.tw_off[0] + k];
+  for (int k = threadIdx.x; k < Ly; k += kPartThreads) twy[k] = c.tw[c.tw_off[1] + k];
+  const C2 *links = c.links + (size_t)blockIdx.x * Lx * Ly * 36;
+  const int Q = Kx * kNF;        // x components of one row
+  const int nx = c.b[0] + 1, ny = c.b[1] + 1;
+  C2 P[NT], S[NT];
+#pragma unroll
+  for (int k = 0; k < NT; k++) P[k] = S[k] = mk<double>(0., 0.);
+  for (int y0 = 0; y0 < Ly; y0 += R) {
+    const int rows = min(R, Ly - y0);
+    // one link a thread: its four packed components
+    for (int l = threadIdx.x; l < rows * Lx * 4; l += kPartThreads) {
+      const C2 *u = links + ((size_t)y0 * Lx * 4 + l) * 9;
+      C2 r[9], v[4];
+#pragma unroll
+      for (int j = 0; j < 9; j++) r[j] = u[j];
+      if constexpr (LOG) {
+        log_components(r, v);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = lin_component(r, q);
+      }
+      C2 *a = A + (size_t)l * 4;
+#pragma unroll
+      for (int q = 0; q < 4; q++) a[(q + l) & 3] = v[q];
+    }
+    __syncthreads();
+    // x: field fastest, then the row, then the pair
+    for (int o = threadIdx.x; o < rows * kNF * nx; o += kPartThreads) {
+      const int f = o % kNF, r = o / kNF % rows, n = o / kNF / rows;
+      const C2 *a = A + (size_t)r * Lx * kNF + f;
+      C2 p = mk<double>(0., 0.), q = p;
+      int w = 0;
+#pragma unroll 4
+      for (int x = 0; x < Lx; x++) {
+        pair_add(a[x * kNF], twx[w], &p, &q);
+        w += n;
+        w -= w >= Lx ? Lx : 0;
+      }
+      C2 *d = X + (size_t)r * Q + f;
+      d[n * kNF] = pair_pos(p, q);
+      if (n && 2 * n != Lx) d[(Kx - n) * kNF] = pair_neg(p, q);
+    }
+    __syncthreads();
+    // y: the sums stay with their threads
+#pragma unroll
+    for (int k = 0; k < NT; k++) {
+      const int o = threadIdx.x + k * kPartThreads;
+      if (o < Q * ny) {
+        const int n = o / Q, col = o - n * Q;
+        int w = (int)((long long)n * y0 % Ly);
+        for (int r = 0; r < rows; r++) {
+          pair_add(X[(size_t)r * Q + col], twy[w], &P[k], &S[k]);
+          w += n;
+          w -= w >= Ly ? Ly : 0;
+        }
+      }
+    }
+    // (the next chunk's x sums follow a barrier, after which X is free)
+  }
+  C2 *out = c.F1 + (size_t)blockIdx.x * Ky * Q;
+#pragma unroll
+  for (int k = 0; k < NT; k++) {
+    const int o = threadIdx.x + k * kPartThreads;
+    if (o < Q * ny) {
+      const int n = o / Q, col = o - n * Q;
+      out[(size_t)n * Q + col] = pair_pos(P[k], S[k]);
+      if (n && 2 * n != Ly) out[(size_t)(Ky - n) * Q + col] = pair_neg(P[k], S[k]);
+    }
+  }
+}
+
+// the kept components of one more axis of `len` elements: in[g][len][C] ->
+// out[g][K][C], thread per column, pair and group g = blockIdx.y
+__global__ void __launch_bounds__(128) k_cut_part(const C2 *in, C2 *out, const C2 *tw, int len,
+                                                  int K, int C) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x, n = blockIdx.z;
+  if (col >= C) return;
+  const C2 *a = in + (size_t)blockIdx.y * len * C + col;
+  C2 p = mk<double>(0., 0.), q = p;
+  int w = 0;
+#pragma unroll 8
+  for (int k = 0; k < len; k++) {
+    pair_add(a[(size_t)k * C], tw[w], &p, &q);
+    w += n;
+    w -= w >= len ? len : 0;
+  }
+  C2 *d = out + (size_t)blockIdx.y * K * C + col;
+  d[(size_t)n * C] = pair_pos(p, q);
+  if (n && 2 * n != len) d[(size_t)(K - n) * C] = pair_neg(p, q);
+}
+
 using CutFn = void (*)(CutCtx);
 
 static CutFn xy4_ct(int lx, int ly, bool log) {
@@ -393,8 +543,10 @@ static std::vector<std::pair<int, CutFn>> zt_ct(int lz, int lt, int lx) {
 
 // per listed momentum i: G[i][mu][9] = A_mu(p) e^{i p_mu / 2} and the
 // p-space error term |sum_mu,j p_mu G_mu,j| / 9 (pspace_landau.c:38-77)
-__global__ void __launch_bounds__(128) k_cut_gather(const C2 *F, int V, int nmom,
-                                                    const int2 *sites,
+// Field (mu, q) of site s is at s ss + (4 mu + q) fs, q counted from mu for the
+// partial transforms (rot).
+__global__ void __launch_bounds__(128) k_cut_gather(const C2 *F, size_t ss, size_t fs, int rot,
+                                                    int nmom, const int2 *sites,
                                                     const C2 *phase,
                                                     const double *pmu, C2 *G,
                                                     double *err) {
@@ -404,11 +556,13 @@ __global__ void __launch_bounds__(128) k_cut_gather(const C2 *F, int V, int nmom
   C2 sum = mk<double>(0., 0.);
 #pragma unroll
   for (int mu = 0; mu < 4; mu++) {
-    const C2 *f = F + (size_t)(mu * 4) * V;
-    const C2 c0p = f[st.x], c0n = f[st.y];
-    const C2 c1p = f[(size_t)V + st.x], c1n = f[(size_t)V + st.y];
-    const C2 c2p = f[2 * (size_t)V + st.x], c2n = f[2 * (size_t)V + st.y];
-    const C2 c3p = f[3 * (size_t)V + st.x], c3n = f[3 * (size_t)V + st.y];
+    auto at = [&](int site, int k) {
+      return F[(size_t)site * ss + (size_t)(4 * mu + ((k + (rot ? mu : 0)) & 3)) * fs];
+    };
+    const C2 c0p = at(st.x, 0), c0n = at(st.y, 0);
+    const C2 c1p = at(st.x, 1), c1n = at(st.y, 1);
+    const C2 c2p = at(st.x, 2), c2n = at(st.y, 2);
+    const C2 c3p = at(st.x, 3), c3n = at(st.y, 3);
     C2 q[9];
     q[0] = mk<double>((c0p.x + c0n.x) / 2., (c0p.y - c0n.y) / 2.);
     q[4] = mk<double>((c0p.y + c0n.y) / 2., -(c0p.x - c0n.x) / 2.);
@@ -554,6 +708,9 @@ struct CutKey {
 struct MomList {
   std::vector<int> mom;     // 4 per momentum, -pi..pi zone
   std::vector<int2> sites;  // 0..2pi-zone sites of p and -p
+  std::vector<int2> box;    // the same in the box of kept components
+  int b[4] = {0, 0, 0, 0};  // largest |n_mu| of the list
+  int K[4] = {1, 1, 1, 1};  // kept components of each axis
   std::vector<C2> phase;    // e^{i p_mu / 2} per momentum and direction
   std::vector<double> pmu;  // 2 sin(p_mu / 2)
   std::vector<double> psq;  // sum_mu pmu^2, 1 below PREC_TOL
@@ -679,6 +836,19 @@ static int build_list(const int L[4], const gfix_cut_info &ci, MomList &ml) {
           ml.psq.push_back(ps < kPrecTol ? 1.0 : ps);
           ml.sites.push_back(make_int2(sp, sn));
         }
+  for (size_t i = 0; i < ml.n(); i++)
+    for (int mu = 0; mu < 4; mu++) ml.b[mu] = std::max(ml.b[mu], std::abs(ml.mom[i * 4 + mu]));
+  for (int mu = 0; mu < 4; mu++) ml.K[mu] = std::min(L[mu], 2 * ml.b[mu] + 1);
+  for (size_t i = 0; i < ml.n(); i++) {
+    int s[2] = {0, 0};
+    for (int mu = 3; mu >= 0; mu--)
+      for (int k = 0; k < 2; k++) {
+        const int m = k ? -ml.mom[i * 4 + mu] : ml.mom[i * 4 + mu];
+        const int r = (m % L[mu] + L[mu]) % L[mu];  // residue, then its place
+        s[k] = s[k] * ml.K[mu] + (r <= ml.b[mu] ? r : ml.K[mu] - (L[mu] - r));
+      }
+    ml.box.push_back(make_int2(s[0], s[1]));
+  }
   return 0;
 }
 
@@ -704,6 +874,7 @@ struct Work {
   bool xy4 = false;  // xy_fn are k_cut_xy4_ct (the Lie fields computed inside)
   std::map<CutKey, MomList> lists;
   const MomList *cur = nullptr;  // list on the device
+  bool part = false;             // its momenta by partial transforms
 
   ~Work() {
     cudaFree(d_links);
@@ -852,6 +1023,18 @@ struct Work {
     return &lists.emplace(k, std::move(ml)).first->second;
   }
 
+  // Partial transforms serve a list whose kept components are at most a
+  // quarter of an xy plane (the fields they leave then fit in d_F, three
+  // times): both passes take 0.197 against 0.459 ms with 81 of 400 components
+  // (20^3 x 40), 0.858 against 1.274 ms with 81 of 1024 (32^3 x 64), but 0.090
+  // against 0.084 ms with 81 of 256 (16^3 x 32).  Their rows must be short
+  // enough for a chunk of them in shared memory.
+  bool partial(const MomList &ml) const {
+    return 4 * ml.K[0] * ml.K[1] <= L[0] * L[1] && L[0] <= 2 * kPartSites &&
+           ml.K[0] * kNF * (ml.b[1] + 1) <= kPartTasks * kPartThreads &&
+           part_smem(L[0], L[1], ml.K[0]) <= 200u * 1024u;
+  }
+
   int upload(const MomList *ml) {
     if (cur == ml) return 0;
     const size_t n = std::max<size_t>(ml->n(), 1);
@@ -879,6 +1062,7 @@ struct Work {
       cap = n;
     }
     cur = nullptr;
+    const bool pt = partial(*ml);
     if (ml->n()) {
       CCK(cudaMemcpyAsync(d_phase, ml->phase.data(), ml->n() * 4 * sizeof(C2),
                           cudaMemcpyHostToDevice, s));
@@ -886,11 +1070,12 @@ struct Work {
                           cudaMemcpyHostToDevice, s));
       CCK(cudaMemcpyAsync(d_psq, ml->psq.data(), ml->n() * sizeof(double),
                           cudaMemcpyHostToDevice, s));
-      CCK(cudaMemcpyAsync(d_sites, ml->sites.data(), ml->n() * sizeof(int2),
+      CCK(cudaMemcpyAsync(d_sites, (pt ? ml->box : ml->sites).data(), ml->n() * sizeof(int2),
                           cudaMemcpyHostToDevice, s));
     }
     CCK(cudaStreamSynchronize(s));
     cur = ml;
+    part = pt;
     return 0;
   }
 
@@ -899,10 +1084,52 @@ struct Work {
     return 0;
   }
 
+  // the kept components of the current list's axes; F3, the last of them,
+  // follows F1 and F2 in d_F
+  PartCtx part_ctx() const {
+    PartCtx p;
+    for (int a = 0; a < 4; a++) {
+      p.L[a] = L[a];
+      p.b[a] = cur->b[a];
+      p.K[a] = cur->K[a];
+      p.tw_off[a] = c.ax[a].tw_off;
+    }
+    const size_t C = (size_t)kNF * p.K[0] * p.K[1];
+    p.links = c.links;
+    p.tw = d_tw;
+    p.F1 = d_F;
+    p.F2 = p.F1 + C * L[2] * L[3];
+    p.F3 = p.F2 + C * p.K[2] * L[3];
+    return p;
+  }
+  template <bool LOG>
+  int part_pxy(const PartCtx &p) {
+    const int tasks = (p.K[0] * kNF * (p.b[1] + 1) + kPartThreads - 1) / kPartThreads;
+    auto f = tasks <= 1 ? k_cut_pxy<LOG, 1> : tasks <= 3 ? k_cut_pxy<LOG, 3>
+                                                         : k_cut_pxy<LOG, kPartTasks>;
+    const size_t sm = part_smem(L[0], L[1], p.K[0]);
+    if (attr(f, sm)) return -1;
+    f<<<L[2] * L[3], kPartThreads, sm, s>>>(p);
+    return 0;
+  }
+  int transform_part(bool log, cudaEvent_t mid) {
+    const PartCtx p = part_ctx();
+    if (log ? part_pxy<true>(p) : part_pxy<false>(p)) return -1;
+    if (mid) cudaEventRecord(mid, s);
+    const int C = kNF * p.K[0] * p.K[1], Cz = C * p.K[2];
+    k_cut_part<<<dim3((C + 127) / 128, L[3], p.b[2] + 1), 128, 0, s>>>(
+        p.F1, p.F2, d_tw + p.tw_off[2], L[2], p.K[2], C);
+    k_cut_part<<<dim3((Cz + 127) / 128, 1, p.b[3] + 1), 128, 0, s>>>(
+        p.F2, p.F3, d_tw + p.tw_off[3], L[3], p.K[3], Cz);
+    count_launches(3);
+    return 0;
+  }
+
   // the transforms of the Lie fields (definition def) of c.links into
   // d_F; `mid` (may be null) is recorded between the xy and the zt pass
-  void transform(int def, cudaEvent_t mid = nullptr) {
+  int transform(int def, cudaEvent_t mid = nullptr) {
     const bool log = def == GFIX_FIELD_LOG;
+    if (part) return transform_part(log, mid);
     const dim3 gxy(xy4 ? 4 : kNF, L[2] * L[3]);
     if (log && !xy4) {
       k_cut_log_pack<<<(unsigned)(((size_t)V * 4 + 127) / 128), 128, 0, s>>>(c);
@@ -930,6 +1157,7 @@ struct Work {
     else
       k_cut_zt<16, false><<<gzt, bd_zt, sm_zt, s>>>(c);
     count_launches(2);
+    return 0;
   }
 
   Norms norms() const {
@@ -943,7 +1171,11 @@ struct Work {
     const int n = (int)cur->n();
     if (n == 0) return;
     const int nb = (n + 127) / 128;
-    k_cut_gather<<<nb, 128, 0, s>>>(d_F, V, n, d_sites, d_phase, d_pmu, d_G, d_err);
+    if (part)
+      k_cut_gather<<<nb, 128, 0, s>>>(part_ctx().F3, kNF, 1, 1, n, d_sites, d_phase, d_pmu, d_G,
+                                      d_err);
+    else
+      k_cut_gather<<<nb, 128, 0, s>>>(d_F, 1, V, 0, n, d_sites, d_phase, d_pmu, d_G, d_err);
     if (dir == GFIX_CUT_GLUON_PROPS)
       k_cut_props<<<nb, 128, 0, s>>>(d_G, n >> 1, d_pmu, d_psq, norms(), d_o0, d_o1);
     else if (dir == GFIX_CUT_EXCEPTIONAL)
@@ -1022,7 +1254,7 @@ static int run(Work *w, const gfix_cut_info *ci, size_t nmom, double *out0,
   if (nmom != ml->n())
     return cfail("%zu momenta given, the cut keeps %zu", nmom, ml->n());
   if (w->upload(ml)) return -1;
-  w->transform(ci->definition);
+  if (w->transform(ci->definition)) return -1;
   w->measure(ci->dir);
   CCK(cudaGetLastError());
   return w->fetch(ci->dir, out0, out1, perr);
@@ -1179,7 +1411,7 @@ int gfix_profile_cuts(const double *d_links, const size_t dims[4], const gfix_cu
   float acc[3] = {0, 0, 0};
   for (int r = 0; r < reps + 1; r++) {
     CCK(cudaEventRecord(ev[0], w->s));
-    w->transform(ci->definition, ev[1]);
+    if (w->transform(ci->definition, ev[1])) return -1;
     CCK(cudaEventRecord(ev[2], w->s));
     w->measure(ci->dir);
     CCK(cudaEventRecord(ev[3], w->s));

@@ -201,3 +201,25 @@ def test_glu_named_cuts_struct_writes_glus_file(lat400, tmp_path, monkeypatch):
     assert _close(got["longitudinal"], ref["longitudinal"], np.abs(ref["transverse"]).max())
     ci.dir = 1  # NON_EXCEPTIONAL: not provided
     assert lib.cuts_struct(sites, ci) == -1
+
+
+@pytest.mark.parametrize("dims,maxmom,field", [
+    ((8, 8, 6, 10), 1, "LINEAR"), ((6, 7, 6, 10), 1, "LOGARITHMIC"), ((16, 16, 16, 16), 4, "LINEAR"),
+    ((24, 24, 12, 12), 4, "LOGARITHMIC"), ((24, 24, 12, 12), 7, "LINEAR"),
+    ((32, 8, 8, 8), 1, "LINEAR"), ((9, 15, 10, 9), 1, "LINEAR"), ((128, 8, 8, 8), 1, "LINEAR")])
+def test_partial_transforms_equal_full_ones(dims, maxmom, field):
+    """A cut that keeps few momenta sums each axis into those alone; the
+    fields at its momenta are the full transforms', which a cut that keeps
+    every momentum takes."""
+    from glu_b200.workload import random_su3
+    V = int(np.prod(dims))
+    U = random_su3(4 * V, np.random.default_rng(6)).reshape(V, 4, 3, 3)
+    few = cuts.CutInfo("FIELDS", "HYPERCUBIC_CUT", field, maxmom=maxmom)
+    every = cuts.CutInfo("FIELDS", "HYPERCUBIC_CUT", field, maxmom=max(dims) ** 2)
+    a, b = cuts.measure(U, dims, few), cuts.measure(U, dims, every)
+    assert len(b["mom"]) == V and 0 < len(a["mom"]) < V
+    at = {tuple(m): i for i, m in enumerate(b["mom"])}
+    w = b["fields"][[at[tuple(m)] for m in a["mom"]]]
+    # sums of V terms of order one
+    assert np.abs(a["fields"] - w).max() < 1e-14 * V
+    assert np.abs(w).max() > 1.0
