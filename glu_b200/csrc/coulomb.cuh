@@ -111,13 +111,6 @@ __device__ __forceinline__ int sbck(const SliceSite &q, const int *L) {
   return q.x[MU] == 0 ? q.i + (L[MU] - 1) * sd : q.i - sd;
 }
 
-// buffer of a ping-pong pair by parity, as a select (a runtime index into
-// the by-value kernel parameter would copy it to local memory)
-template <typename T>
-__device__ __forceinline__ T *pick(T *const (&b)[2], int p) {
-  return p ? b[1] : b[0];
-}
-
 template <typename R>
 __device__ __forceinline__ void load9(const cx<R> *p, int V, int s, cx<R> *u) {
 #pragma unroll
