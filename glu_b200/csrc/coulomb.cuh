@@ -122,71 +122,60 @@ __device__ __forceinline__ void store9(cx<R> *p, int V, int s, const cx<R> *u) {
   for (int e = 0; e < 9; e++) p[(size_t)e * V + s] = u[e];
 }
 
-// rotated link g(a) U g(b)^dag of the reference's gtransform_local
-template <typename R>
-__device__ __forceinline__ void rotated(const CCtx<R> &c, int mu, int s_link,
-                                        int sa, int sb, cx<R> *C) {
-  cx<R> A[9], B[9];
-  load_link(c.U, c.V, mu, s_link, C);
-  load9(c.g, c.V, sa, A);
-  load9(c.g, c.V, sb, B);
-  gtransform(A, C, B);
-}
-
-// Hermitian short form of the rotated link (5 entries), formed in the
-// arithmetic type CT from links and g stored in R
-template <typename R>
-struct HShort {
-  R h0, h3;
-  cx<R> h1, h2, h4;
-};
-// rotated link g(a) U g(b)^dag in the arithmetic type CT
-template <typename R, typename CT>
-__device__ __forceinline__ void rotated_ct(const CCtx<R> &c, int mu, int s_link,
-                                           int sa, int sb, cx<CT> *C) {
-  auto up = [](cx<R> a) { return mk<CT>((CT)a.x, (CT)a.y); };
-  cx<CT> A[9], B[9];
-  {
-    cx<R> t[9];
-    load_link(c.U, c.V, mu, s_link, t);
-#pragma unroll
-    for (int e = 0; e < 9; e++) C[e] = up(t[e]);
-    load9(c.g, c.V, sa, t);
-#pragma unroll
-    for (int e = 0; e < 9; e++) A[e] = up(t[e]);
-    load9(c.g, c.V, sb, t);
-#pragma unroll
-    for (int e = 0; e < 9; e++) B[e] = up(t[e]);
-  }
-  gtransform(A, C, B);
-}
-
-template <typename R, typename CT>
-__device__ __forceinline__ HShort<CT> rotated_herm(const CCtx<R> &c, int mu,
-                                                   int s_link, int sa, int sb) {
-  cx<CT> C[9];
-  rotated_ct<R, CT>(c, mu, s_link, sa, sb, C);
-  HShort<CT> h;
-  herm_short(C, h.h0, h.h1, h.h2, h.h3, h.h4);
-  return h;
+template <typename CT, typename R>
+__device__ __forceinline__ cx<CT> up_to(cx<R> a) {
+  return mk<CT>((CT)a.x, (CT)a.y);
 }
 
 // ---------------------------------------------------------------------
-// derivative on the rotated links, packed like the Landau fields
-// (steep_deriv_CG, src/Gfix/CFACG.c:91-163)
+// derivative on the rotated links W_i(x) = g(x) U_i(x) g(x+i)^dag, packed like
+// the Landau fields (steep_deriv_CG, src/Gfix/CFACG.c:91-163).  Only the
+// traceless anti-Hermitian part of sum_i W_i(x-i) - W_i(x) enters, and W and
+// -W^dag have the same one, so with
+//   S(x) = sum_i U_i(x) g(x+i)^dag + (g(x-i) U_i(x-i))^dag
+// it is that of -g(x) S(x): one product for each of the six links and one
+// with g(x), in place of two for each.  At 32^3 x 64, FP64: 0.324 -> 0.215 ms
+// (0.74 of the copy bandwidth on its algorithmic bytes; four blocks per SM,
+// three take 0.228 ms), FP32 storage 0.236 -> 0.162 ms.
 template <typename R, typename CT, int MU>
 __device__ __forceinline__ void cderiv_dir(const CCtx<R> &c, const SliceSite &q,
-                                           int off, CT &s0, cx<CT> &s1,
-                                           cx<CT> &s2, CT &s3, cx<CT> &s4) {
+                                           int off, cx<CT> *S) {
   const int it = sfwd<MU>(q, c.L), bk = sbck<MU>(q, c.L);
-  // g(i) U(i) g(i+mu)^dag and g(i-mu) U(i-mu) g(i)^dag
-  const HShort<CT> b = rotated_herm<R, CT>(c, MU, off + q.i, off + q.i, off + it);
-  const HShort<CT> a = rotated_herm<R, CT>(c, MU, off + bk, off + bk, off + q.i);
-  s0 += a.h0 - b.h0;
-  s1 = cadd(s1, csub(a.h1, b.h1));
-  s2 = cadd(s2, csub(a.h2, b.h2));
-  s3 += a.h3 - b.h3;
-  s4 = cadd(s4, csub(a.h4, b.h4));
+  cx<R> t[9];
+  cx<CT> U[9], G[9];
+  load_link(c.U, c.V, MU, off + q.i, t);
+#pragma unroll
+  for (int e = 0; e < 9; e++) U[e] = up_to<CT>(t[e]);
+  if constexpr (sizeof(CT) != sizeof(R)) complete_col2(U);
+  load9(c.g, c.V, off + it, t);
+#pragma unroll
+  for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t[e]);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        S[3 * i + j] = cmaddc(S[3 * i + j], U[3 * i + k], G[3 * j + k]);
+  // P = g(x-i) U(x-i): the first two columns, the third completed
+  cx<R> r0[3], r1[3];
+  cx<CT> u0[3], u1[3], p0[3], p1[3];
+  load_cols(c.U, c.V, MU, off + bk, r0, r1);
+#pragma unroll
+  for (int r = 0; r < 3; r++) u0[r] = up_to<CT>(r0[r]), u1[r] = up_to<CT>(r1[r]);
+  load9(c.g, c.V, off + bk, t);
+#pragma unroll
+  for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t[e]);
+  mat_vec(p0, G, u0);
+  mat_vec(p1, G, u1);
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    S[r] = cadd(S[r], conjg(p0[r]));
+    S[3 + r] = cadd(S[3 + r], conjg(p1[r]));
+  }
+  S[6] = cadd(S[6], conjg(cdet(p0[1], p1[2], p0[2], p1[1])));
+  S[7] = cadd(S[7], conjg(cdet(p0[2], p1[0], p0[0], p1[2])));
+  S[8] = cadd(S[8], conjg(cdet(p0[0], p1[1], p0[1], p1[0])));
 }
 
 // CT: arithmetic type.  With FP32 storage a slice below theta = hp_below is
@@ -202,18 +191,35 @@ __global__ void __launch_bounds__(kCoulThreads, 4) k_cderiv(CCtx<R> c, int sel) 
   if (i >= c.Lcu) return;
   const SliceSite q = slice_site(i, c.L);
   const int off = t * c.Lcu;
-  CT s0 = 0, s3 = 0;
-  cx<CT> s1 = mk<CT>(0, 0), s2 = mk<CT>(0, 0), s4 = mk<CT>(0, 0);
-  cderiv_dir<R, CT, 0>(c, q, off, s0, s1, s2, s3, s4);
-  cderiv_dir<R, CT, 1>(c, q, off, s0, s1, s2, s3, s4);
-  cderiv_dir<R, CT, 2>(c, q, off, s0, s1, s2, s3, s4);
-  // pack: in0 = i Re s0 - Re s3, in_k = i Re s_k - Im s_k (CFACG.c:144-150)
+  cx<CT> S[9], G[9], M[9];
+#pragma unroll
+  for (int e = 0; e < 9; e++) S[e] = mk<CT>(0, 0);
+  cderiv_dir<R, CT, 0>(c, q, off, S);
+  cderiv_dir<R, CT, 1>(c, q, off, S);
+  cderiv_dir<R, CT, 2>(c, q, off, S);
+  {
+    cx<R> t9[9];
+    load9(c.g, c.V, off + i, t9);
+#pragma unroll
+    for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t9[e]);
+  }
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      M[3 * r + k] = cmadd(cmadd(cmul(G[3 * r], S[k]), G[3 * r + 1], S[3 + k]),
+                           G[3 * r + 2], S[6 + k]);
+  CT s0, s3;
+  cx<CT> s1, s2, s4;
+  herm_short(M, s0, s1, s2, s3, s4);
+  // pack: in0 = i Re s0 - Re s3, in_k = i Re s_k - Im s_k of -g S
+  // (CFACG.c:144-150)
   cx<R> *f = pick(c.fb, c.st->parity);
   const size_t V = c.V, s = off + i;
-  f[s] = mk<R>((R)-s3, (R)s0);
-  f[V + s] = mk<R>((R)-s1.y, (R)s1.x);
-  f[2 * V + s] = mk<R>((R)-s2.y, (R)s2.x);
-  f[3 * V + s] = mk<R>((R)-s4.y, (R)s4.x);
+  f[s] = mk<R>((R)s3, (R)-s0);
+  f[V + s] = mk<R>((R)s1.y, (R)-s1.x);
+  f[2 * V + s] = mk<R>((R)s2.y, (R)-s2.x);
+  f[3 * V + s] = mk<R>((R)s4.y, (R)-s4.x);
 }
 
 // The sums of the accelerated field, insum (sum_DER2 / sum_PR, one norm) and
@@ -242,13 +248,15 @@ __device__ __forceinline__ void cdir(const cx<R> *in, const cx<R> *so, R beta,
 // every live slice, and the line-search probes of line_search_Coulomb
 // (src/Gfix/line_search.c:141-271) at 0.17 and 0.34 as differences to the
 // alpha = 0 value; each link counted once (the forward links of every site,
-// the same set the reference's draughtboard visits).  Per link the rotated
-// link C = g(x) U g(x+mu)^dag is formed once and serves both probes; the
-// probe gauge matrices of the site itself wait in shared memory.
+// the same set the reference's draughtboard visits).  Per link the first
+// two columns of the rotated link g(x) U g(x+mu)^dag are formed once and serve
+// both probes (probe_trace); the probe gauge matrices of the site itself wait
+// in shared memory.  At 32^3 x 64: 0.453 -> 0.403 ms in FP64, bound by its
+// arithmetic at three blocks per SM, 0.300 -> 0.269 ms in FP32 at four.
 // CT: arithmetic type of the probes (FP64 for FP32 storage below hp_below,
 // as in k_cderiv); `sel` picks the slices of this variant.
 template <typename R, typename CT = R>
-__global__ void __launch_bounds__(kCoulThreads, 3) k_cprobe(CCtx<R> c, int sel) {
+__global__ void __launch_bounds__(kCoulThreads, sizeof(CT) == 4 ? 4 : 3) k_cprobe(CCtx<R> c, int sel) {
   __shared__ cx<CT> sA[2][9][kCoulThreads];
   const int t = blockIdx.y;
   if (arith_skip(sel, c.sl[t].tr, c.cs->hp_below)) return;
@@ -283,18 +291,38 @@ __global__ void __launch_bounds__(kCoulThreads, 3) k_cprobe(CCtx<R> c, int sel) 
 #pragma unroll 1
       for (int mu = 0; mu < 3; mu++) {
         const int it = sfwd_rt(q, c.L, mu);
-        cx<CT> Cd[9];
-        rotated_ct<R, CT>(c, mu, off + i, off + i, off + it, Cd);
-        const CT t0 = Cd[0].x + Cd[4].x + Cd[8].x;
+        // the first two columns of C = g(x) U g(x+mu)^dag
+        cx<CT> w0[3], w1[3];
+        {
+          cx<R> t9[9];
+          cx<CT> U[9], G[9], b0[3], b1[3];
+          load_link(c.U, c.V, mu, off + i, t9);
+#pragma unroll
+          for (int e = 0; e < 9; e++) U[e] = up(t9[e]);
+          if constexpr (sizeof(CT) != sizeof(R)) complete_col2(U);
+#pragma unroll
+          for (int e = 0; e < 6; e++) G[e] = up(c.g[(size_t)e * c.V + off + it]);
+#pragma unroll
+          for (int r = 0; r < 3; r++) {
+            b0[r] = cmaddc(cmaddc(cmulc(U[3 * r], G[0]), U[3 * r + 1], G[1]), U[3 * r + 2], G[2]);
+            b1[r] = cmaddc(cmaddc(cmulc(U[3 * r], G[3]), U[3 * r + 1], G[4]), U[3 * r + 2], G[5]);
+          }
+          load9(c.g, c.V, off + i, t9);
+#pragma unroll
+          for (int e = 0; e < 9; e++) G[e] = up(t9[e]);
+          mat_vec(w0, G, b0);
+          mat_vec(w1, G, b1);
+        }
+        const CT t0 = re_tr_cols(w0, w1);
         cx<R> fy[4];
         cdir(in, so, beta, sdstep, (size_t)off + it, (size_t)c.V, fy);
+        const ProbeDir<CT> p = probe_dir(up(fy[0]), up(fy[1]), up(fy[2]), up(fy[3]));
 #pragma unroll 1
         for (int k = 0; k < 2; k++) {
-          cx<CT> A[9], Bm[9];
+          cx<CT> A[9];
 #pragma unroll
           for (int e = 0; e < 9; e++) A[e] = sA[k][e][threadIdx.x];
-          set_gauge(Bm, up(fy[0]), up(fy[1]), up(fy[2]), up(fy[3]), k ? al1 : al0);
-          d[k] += re_tr_abc_dag(A, Cd, Bm) - t0;
+          d[k] += probe_trace(A, w0, w1, p, k ? al1 : al0) - t0;
         }
       }
       v[0] = d[0];
