@@ -19,52 +19,6 @@
 
 namespace gfix {
 
-// PREC_TOL (GLU_definitions.h:359-363): NC 1e-14 in double, NC 1e-6 in
-// single precision builds
-constexpr double kPrecTol = 3 * 1.0E-14;
-constexpr double kPrecTolSingle = 3 * 1.0E-6;
-constexpr int kCoulThreads = 128;
-
-enum SliceMode : int { SL_RUN = 0, SL_DONE = 1 };
-
-struct Slice {
-  double tr, inold, insum, sumconj, beta, alpha;
-  long long iter;     // steps of the current run (GLU's loc_iters)
-  long long tot;      // GLU's tot_iters of steep_fix
-  int sd;             // next step is an SD step
-  int use_ls;
-  int mode;           // SL_RUN / SL_DONE
-  int control;        // random restarts so far
-  int reunit;         // maintenance: reunitarise g_t and check it
-  int randomize;      // maintenance: random restart of g_t
-  int bad;            // set when the unitarity check fails
-  int trans;          // GLU's trans_flag: survives a continuation run
-  int traj_len;
-  double best_tr;     // stall rule (mixed-precision FP32 phase)
-  long long since_best;
-};
-
-struct CoulState {
-  double gf_alpha, acc, cg_tol;
-  long long max_iters;
-  int facg;           // 1 FACG, 0 FASD
-  int sd_fixed;       // GLU_GFIX_SD semantics
-  int active;         // slices still running
-  int nslices;
-  unsigned long long seed;
-  int traj_cap;       // per slice
-  double *traj;       // [nslices][traj_cap]
-  int *done_mask;     // [nslices], 1 once a slice has finished (FFT passes skip it)
-  double prec_tol;    // PREC_TOL of the unitarity check
-  double hp_below;    // FP32 storage: FP64 arithmetic for slices below this theta
-  // stall rule of a mixed-precision FP32 phase (stall_window 0: off): a
-  // slice whose best theta is below stall_floor ends its run after
-  // stall_window iterations without a 10% improvement on it, or on a jump
-  // above blowup x it; the FP64 phase then continues it
-  long long stall_window;
-  double stall_floor, blowup;
-};
-
 template <typename R>
 struct CCtx {
   cx<R> *U;           // links SoA [4][9][V]
@@ -75,6 +29,7 @@ struct CCtx {
   CoulState *cs;
   Slice *sl;
   double *part;       // [nslices][nbs][2]
+  unsigned *tick;     // a ticket for each slice, zero between kernels
   int L[4];
   int V, Lcu, nbs;
 };
@@ -259,13 +214,12 @@ template <typename R, typename CT = R>
 __global__ void __launch_bounds__(kCoulThreads, sizeof(CT) == 4 ? 4 : 3) k_cprobe(CCtx<R> c, int sel) {
   __shared__ cx<CT> sA[2][9][kCoulThreads];
   const int t = blockIdx.y;
-  if (arith_skip(sel, c.sl[t].tr, c.cs->hp_below)) return;
-  double v[2] = {0.0, 0.0};
   const Slice &S = c.sl[t];
-  const bool live = S.mode != SL_DONE;
-  const bool probes = live && S.use_ls;
+  if (S.mode == SL_DONE || arith_skip(sel, S.tr, c.cs->hp_below)) return;
+  double v[2] = {0.0, 0.0};
+  const bool probes = S.use_ls;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (live && i < c.Lcu) {
+  if (i < c.Lcu) {
     const int par = c.st->parity, spar = c.st->sparity;
     const cx<R> *in = pick(c.fb, par), *so = pick(c.sb, spar);
     cx<R> *sn = pick(c.sb, spar ^ 1);
@@ -336,10 +290,11 @@ __global__ void __launch_bounds__(kCoulThreads, sizeof(CT) == 4 ? 4 : 3) k_cprob
 // src/Gfix/line_search.c:101-115)
 template <typename R>
 __global__ void __launch_bounds__(kCoulThreads) k_cupdate(CCtx<R> c) {
-  const int t = blockIdx.y;
+  // (from the last site to the first, as k_update)
+  const int t = gridDim.y - 1 - blockIdx.y;
   const Slice &S = c.sl[t];
   if (S.mode == SL_DONE) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= c.Lcu) return;
   const size_t V = c.V, s = (size_t)t * c.Lcu + i;
   const cx<R> *d = pick(c.sb, c.st->sparity ^ 1);
@@ -365,185 +320,104 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   return z ^ (z >> 31);
 }
 
+// what = 0: reunitarise and check, then the end of a run of the slices that
+// have ended theirs; what = 1: random restarts, and the in / in_old and sn
+// ping-pong after every step.  Few slices need either in any step, so the
+// grid holds kMaintBlocks blocks a slice, which loop over its sites (a block
+// for every 128 sites returned at once, but cost 0.14 ms a launch at
+// 64^3 x 128).
+constexpr int kMaintBlocks = 8;
+
 template <typename R>
 __global__ void __launch_bounds__(kCoulThreads) k_cmaint(CCtx<R> c, int what) {
+  if (c.st->done) return;
   const int t = blockIdx.y;
   Slice &S = c.sl[t];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c.Lcu || S.mode == SL_DONE) return;
-  const int s = t * c.Lcu + i;
-  if (what == 0 && S.reunit) {
-    cx<R> G[9];
-    load9(c.g, c.V, s, G);
-    gram_reunit(G);
-    store9(c.g, c.V, s, G);
-    double sum = 0.0;
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (what == 1 && t == 0 && i0 == 0) {
+    c.st->parity ^= 1;
+    c.st->sparity ^= 1;
+  }
+  if (S.mode == SL_DONE) return;
+  if (what == 0 && S.sd == -1) {
+    if (S.reunit)
+      for (int i = i0; i < c.Lcu; i += step) {
+        const int s = t * c.Lcu + i;
+        cx<R> G[9];
+        load9(c.g, c.V, s, G);
+        gram_reunit(G);
+        store9(c.g, c.V, s, G);
+        double sum = 0.0;
 #pragma unroll
-    for (int e = 0; e < 9; e++) sum += (double)G[e].x * G[e].x + (double)G[e].y * G[e].y;
-    const double lim = (double)(S.iter > 0 ? S.iter : 1) * c.cs->prec_tol;
-    if (fabs(sum - 3.0) > lim) atomicOr(&S.bad, 1);
+        for (int e = 0; e < 9; e++) sum += (double)G[e].x * G[e].x + (double)G[e].y * G[e].y;
+        const double lim = (double)(S.iter > 0 ? S.iter : 1) * c.cs->prec_tol;
+        if (fabs(sum - 3.0) > lim) atomicOr(&S.bad, 1);
+      }
+    if (arrive_last(c.tick + t, gridDim.x) && threadIdx.x == 0)
+      apply_slice(c.cs, c.sl, c.st, t, C_END2, 0.0, 0.0, (double)c.Lcu);
   } else if (what == 1 && S.randomize) {
-    cx<R> G[9];
-    unsigned long long h = mix64(c.cs->seed ^ mix64(((unsigned long long)t << 40) ^
-                                                    ((unsigned long long)S.control << 32) ^
-                                                    (unsigned long long)i));
+    for (int i = i0; i < c.Lcu; i += step) {
+      cx<R> G[9];
+      unsigned long long h = mix64(c.cs->seed ^ mix64(((unsigned long long)t << 40) ^
+                                                      ((unsigned long long)S.control << 32) ^
+                                                      (unsigned long long)i));
 #pragma unroll
-    for (int e = 0; e < 9; e++) {
-      h = mix64(h);
-      const double u1 = ((h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-      h = mix64(h);
-      const double u2 = ((h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-      const double rad = sqrt(-2.0 * log(u1));
-      G[e] = mk<R>((R)(rad * cospi(2.0 * u2)), (R)(rad * sinpi(2.0 * u2)));
+      for (int e = 0; e < 9; e++) {
+        h = mix64(h);
+        const double u1 = ((h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
+        h = mix64(h);
+        const double u2 = ((h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
+        const double rad = sqrt(-2.0 * log(u1));
+        G[e] = mk<R>((R)(rad * cospi(2.0 * u2)), (R)(rad * sinpi(2.0 * u2)));
+      }
+      gram_reunit(G);
+      store9(c.g, c.V, t * c.Lcu + i, G);
     }
-    gram_reunit(G);
-    store9(c.g, c.V, s, G);
   }
 }
 
-enum CoulOp : int { C_SUMS = 0, C_PROBES = 1, C_END1 = 2, C_END2 = 3 };
-
 // one warp per slice: fixed-order sums of the slice's partials (each lane
-// a strided subset in order, then a fixed shuffle tree), and GLU's control
-// flow of steep_step_FACG / _FASD and steep_fix (src/Gfix/CFACG.c:285-529)
-// on lane 0.
-// Partials: C_SUMS reads the inverse xy FFT pass's per-plane pairs (plane
-// index field * nplanes + t * lz + z), C_PROBES the probe kernel's per-block
-// pairs (t * nbs + block).
+// a strided subset in order, then a fixed shuffle tree), then the scalar step
+// on lane 0.  Partials: C_SUMS reads the inverse xy pass's pairs (`bps` blocks
+// of the slice in each field, field-major), C_PROBES the probe kernel's
+// per-block pairs (t * nbs + block).  C_PROBES also ends the step (C_END1: the
+// update that follows reads neither).  Tickets in those kernels in place of
+// these launches cost more than they saved (probes 0.403 -> 0.442 ms at 32^3
+// x 64): their grids must have a block for every 128 sites of each slice, as
+// any number of slices may be left.
 constexpr int kCScalarSlices = 4;  // slices (warps) per block
 
 __global__ void __launch_bounds__(32 * kCScalarSlices)
-    k_cscalar(CoulState *cs, Slice *sl, const double *part, int nbs, int lz,
-              int nplanes, int op, double Lcu, DevState *st) {
+    k_cscalar(CoulState *cs, Slice *sl, const double *part, int nbs, int bps, int op,
+              double Lcu, DevState *st) {
   const int t = blockIdx.x * kCScalarSlices + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (t < cs->nslices) {
-    Slice &S = sl[t];
-    if (S.mode != SL_DONE) {
-      double a0 = 0.0, a1 = 0.0;
-      if (op == C_SUMS) {
-        const int n = 4 * lz;  // (field, z) pairs, field-major
-        for (int j = lane; j < n; j += 32) {
-          const int f = j / lz, z = j % lz;
-          const size_t b = (size_t)f * nplanes + (size_t)t * lz + z;
-          a0 += part[2 * b];
-          a1 += part[2 * b + 1];
-        }
-      } else if (op == C_PROBES) {
-        constexpr int kU = 4;
-        for (int b0 = lane; b0 < nbs; b0 += 32 * kU) {
-          double x0[kU], x1[kU];
+  if (t >= cs->nslices || sl[t].mode == SL_DONE) return;
+  const size_t np = (size_t)bps * cs->nslices;
+  const int n = op == C_SUMS ? 4 * bps : nbs;
+  double a0 = 0.0, a1 = 0.0;
+  constexpr int kU = 4;
+  for (int b0 = lane; b0 < n; b0 += 32 * kU) {
+    double x0[kU], x1[kU];
 #pragma unroll
-          for (int k = 0; k < kU; k++) {
-            const int b = b0 + 32 * k;
-            x0[k] = b < nbs ? part[2 * ((size_t)t * nbs + b)] : 0.0;
-            x1[k] = b < nbs ? part[2 * ((size_t)t * nbs + b) + 1] : 0.0;
-          }
+    for (int k = 0; k < kU; k++) {
+      const int b = b0 + 32 * k;
+      const size_t i = op == C_SUMS ? (b / bps) * np + (size_t)t * bps + b % bps
+                                    : (size_t)t * nbs + b;
+      x0[k] = b < n ? part[2 * i] : 0.0;
+      x1[k] = b < n ? part[2 * i + 1] : 0.0;
+    }
 #pragma unroll
-          for (int k = 0; k < kU; k++) {
-            a0 += x0[k];
-            a1 += x1[k];
-          }
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        a0 += __shfl_down_sync(0xffffffffu, a0, o);
-        a1 += __shfl_down_sync(0xffffffffu, a1, o);
-      }
-      if (lane != 0) return;
-      switch (op) {
-        case C_SUMS: {
-          S.insum = a0;
-          S.sumconj = a1;
-          S.tr = a0 / (3.0 * Lcu);  // GFNORM_COULOMB
-          if (S.sd) {
-            S.inold = a0;
-            S.beta = 0.0;
-            // FACG's SD start always searches (CFACG.c:318); FASD steps
-            // search unless GLU_GFIX_SD (CFACG.c:270-280)
-            S.use_ls = cs->facg ? 1 : !cs->sd_fixed;
-          } else {
-            const double b = S.sumconj / S.inold;
-            double beta = (b < 0.0) ? 0.0 : b;
-            if (S.tr < cs->cg_tol) beta = S.insum / S.inold;
-            S.beta = beta;
-            S.inold = S.insum;
-            S.use_ls = S.tr > cs->cg_tol;
-          }
-          if (cs->traj && S.traj_len < cs->traj_cap)
-            cs->traj[(size_t)t * cs->traj_cap + S.traj_len++] = S.tr;
-          break;
-        }
-        case C_PROBES: {
-          if (S.use_ls) {
-            const double al[3] = {0.0, 0.17, 0.34};
-            const double f[3] = {0.0, -a0, -a1};
-            S.alpha = approx_minimum(al, f);
-          } else {
-            S.alpha = cs->gf_alpha;
-          }
-          break;
-        }
-        case C_END1: {
-          S.reunit = 0;
-          S.bad = 0;
-          S.randomize = 0;
-          if (cs->facg && S.sd) {
-            S.sd = 0;  // the SD start is not counted
-            break;
-          }
-          S.iter++;
-          if (cs->stall_window > 0 && S.tr > cs->acc) {
-            if (S.tr < 0.9 * S.best_tr) {
-              S.best_tr = S.tr;
-              S.since_best = 0;
-            } else {
-              S.since_best++;
-            }
-            if (S.best_tr < cs->stall_floor &&
-                (S.since_best >= cs->stall_window || S.tr > cs->blowup * S.best_tr)) {
-              S.sd = -1;  // ends the run, no restart: the FP64 phase goes on
-              break;
-            }
-          }
-          if ((S.tr > cs->acc) && (S.iter < cs->max_iters)) break;
-          S.reunit = S.tr < cs->acc;  // run ended: adequate_solution first
-          S.sd = -1;                  // marks "ended" for C_END2
-          break;
-        }
-        case C_END2: {
-          if (S.sd != -1) break;
-          const long long loc = S.iter;
-          const bool fin = isfinite(S.tr);
-          if (S.bad) S.trans = 1;
-          S.sd = 1;
-          S.iter = 0;
-          if (loc >= cs->max_iters) {
-            if (S.tr < 1E4 * cs->acc && fin) {  // continuation run
-              S.tot += loc;
-              break;
-            }
-            if (S.tr > cs->acc || !fin) S.trans = 1;
-          }
-          if (S.control < 8 && S.trans) {  // random restart
-            S.randomize = 1;
-            S.trans = 0;
-            S.tot += loc;
-            S.control++;
-            break;
-          }
-          S.tot += loc;
-          S.iter = loc;
-          S.mode = SL_DONE;
-          cs->done_mask[t] = 1;
-          // the slice that ends last stops the whole sequence
-          if (atomicSub(&cs->active, 1) == 1) st->done = 1;
-          break;
-        }
-      }
+    for (int k = 0; k < kU; k++) {
+      a0 += x0[k];
+      a1 += x1[k];
     }
   }
+  a0 = warp_sum(a0);
+  a1 = warp_sum(a1);
+  if (lane != 0) return;
+  apply_slice(cs, sl, st, t, op, a0, a1, Lcu);
+  if (op == C_PROBES) apply_slice(cs, sl, st, t, C_END1, 0.0, 0.0, Lcu);
 }
 
 // the slice transforms of Coulomb_FA (gtransform_slice, src/Gfix/gtrans.c:
@@ -614,13 +488,6 @@ __global__ void k_cexport_slice(const cx<double> *g, double2 *out, int V,
     const cx<double> v = g[(size_t)e * V + (size_t)t * Lcu + i];
     out[(size_t)e * Lcu + i] = make_double2(v.x, v.y);
   }
-}
-
-// in / in_old and sn ping-pong after every step of every live slice
-__global__ void k_cflip(DevState *st) {
-  if (st->done) return;
-  st->parity ^= 1;
-  st->sparity ^= 1;
 }
 
 template <typename R>

@@ -11,7 +11,7 @@
 template <typename R, int LX, int LY>
 __global__ void __launch_bounds__(ct_threads(LX *LY), ct_minb(LX *LY))
     k_fft_xy_ct(Ctx<R> c, int bwd, int prsum) {
-  if (c.st->done) return;
+  if (xy_done(c, bwd)) return;
   if (c.skip && c.skip[blockIdx.x / c.L[2]]) return;  // finished slice
   constexpr int P = LX + 1, N = LX * LY, BD = ct_threads(N);
   constexpr int EPT = (N + BD - 1) / BD;
@@ -55,9 +55,8 @@ __global__ void __launch_bounds__(ct_threads(LX *LY), ct_minb(LX *LY))
     }
   }
   if (prsum) {
-    block_sum_store<2>(v, c.part + 2 * (blockIdx.y * gridDim.x + blockIdx.x));
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0)
-      c.st->nblocks = gridDim.x * gridDim.y;
+    xy_sums_begin<BD % 32 != 0>(c, v);
+    xy_sums<BD % 32 != 0>(c, v);
   }
 }
 

@@ -17,9 +17,35 @@ __device__ __forceinline__ void stage_twiddles(cx<R> *dst, const cx<R> *src,
   for (int k = threadIdx.x; k < n; k += blockDim.x) dst[k] = src[k];
 }
 
+// has the run finished?  The forward pass, the first kernel after the
+// derivative, then calls off the update
+template <typename R>
+__device__ __forceinline__ bool xy_done(const Ctx<R> &c, bool bwd) {
+  if (!c.st->done) return false;
+  if (!bwd && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) c.st->upd = 0;
+  return true;
+}
+
+// the sums of an inverse xy pass: beta of the run (Landau); Coulomb's are
+// added by slice in k_cscalar, one pair for each block
+template <bool RAGGED, typename R>
+__device__ __forceinline__ void xy_sums_begin(const Ctx<R> &c, double (&v)[2]) {
+  const unsigned np = gridDim.x, b = blockIdx.y * np + blockIdx.x;
+  if (c.ndim == 4)
+    grid_sum_begin<RAGGED>(v, c.part, c.tick, b, 4 * np);
+  else
+    block_sum_store<2, RAGGED>(v, c.part + 2 * (size_t)b);
+}
+template <bool RAGGED, typename R>
+__device__ __forceinline__ void xy_sums(const Ctx<R> &c, double (&v)[2]) {
+  const unsigned np = gridDim.x, b = blockIdx.y * np + blockIdx.x;
+  if (c.ndim == 4 && grid_sum<RAGGED>(v, c.part, c.tick, b, 4 * np))
+    apply_scalar(c.st, OP_PR, v[0], v[1], (double)c.V);
+}
+
 template <typename R, int PT, bool ODD>
 __global__ void __launch_bounds__(512, 2) k_fft_xy(Ctx<R> c, int bwd, int prsum) {
-  if (c.st->done) return;
+  if (xy_done(c, bwd)) return;
   if (c.skip && c.skip[blockIdx.x / c.L[2]]) return;  // finished slice
   extern __shared__ unsigned char smem_raw[];
   __shared__ FftAxis s_ax[2];
@@ -75,9 +101,8 @@ __global__ void __launch_bounds__(512, 2) k_fft_xy(Ctx<R> c, int bwd, int prsum)
     }
   }
   if (prsum) {
-    block_sum_store<2>(v, c.part + 2 * (blockIdx.y * gridDim.x + blockIdx.x));
-    if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0)
-      c.st->nblocks = gridDim.x * gridDim.y;
+    xy_sums_begin<false>(c, v);
+    xy_sums<false>(c, v);
   }
 }
 

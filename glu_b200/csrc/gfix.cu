@@ -54,6 +54,14 @@ static int fail(const char *fmt, ...) {
 
 #define LAUNCHED(n) g_launches.fetch_add((n), std::memory_order_relaxed)
 
+// one counted launch
+template <typename... P, typename... A>
+static void launch(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                   A... a) {
+  k<<<grid, threads, smem, s>>>(P(a)...);
+  LAUNCHED(1);
+}
+
 // kernels launched by the other translation units of the library
 void count_launches(unsigned long long n) { LAUNCHED(n); }
 
@@ -154,6 +162,7 @@ class Engine {
   cudaStream_t s = nullptr;
   DevState *d_st = nullptr, *h_st = nullptr;
   double *d_part = nullptr, *d_cs = nullptr, *d_traj = nullptr;
+  unsigned *d_tick = nullptr;
   cx<F> *d_tw = nullptr, *d_F = nullptr;
   cx<R> *d_U = nullptr, *d_G = nullptr;
   double *d_aos = nullptr;  // AoS FP64 staging (only FP64 engines)
@@ -201,6 +210,7 @@ class Engine {
     cudaFree(d_st);
     cudaFreeHost(h_st);
     cudaFree(d_part);
+    cudaFree(d_tick);
     cudaFree(d_cs);
     cudaFree(d_traj);
     cudaFree(d_tw);
@@ -320,9 +330,16 @@ class Engine {
     g_xy = dim3(V / (c.L[0] * c.L[1]), 4);
     nb_site = (V + kSiteThreads - 1) / kSiteThreads;
     const size_t nparts =
-        std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y) + 1024;
-    CK(cudaMalloc(&d_part, nparts * 2 * sizeof(double)));
+        std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y);
+    const size_t groups = tick_groups((unsigned)nparts);
+    CK(cudaMalloc(&d_part, (nparts + groups) * 2 * sizeof(double)));
     c.part = d_part;
+    // the groups' tickets and the grid's, then one for each time slice
+    const size_t ntick = 1 + groups + c.L[3];
+    CK(cudaMalloc(&d_tick, ntick * sizeof(unsigned)));
+    CK(cudaMemset(d_tick, 0, ntick * sizeof(unsigned)));
+    c.tick = d_tick;
+    c.ctick = d_tick + 1 + groups;
     CK(cudaMalloc(&d_st, sizeof(DevState)));
     CK(cudaMallocHost(&h_st, sizeof(DevState)));
     memset(h_st, 0, sizeof(DevState));
@@ -490,14 +507,22 @@ class Engine {
   }
 
   // --- launch sequences ------------------------------------------------
-  void scalar(int op, int nv) {
-    k_scalar<<<1, kScalarThreads, 0, s>>>(d_st, d_part, op, nv, (double)V);
-    LAUNCHED(1);
+  // the blocks of a kernel over the sites: as many as the SMs hold at once
+  template <typename K>
+  int fill(K k, bool whole = false) {
+    int &n = resident[(const void *)k];
+    if (n == 0) {
+      int per = 0, dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kSiteThreads, 0);
+      n = std::max(1, per * sms);
+    }
+    return whole ? n : std::min(n, nb_site);
   }
+  std::map<const void *, int> resident;
   void theta(int op) {
-    k_deriv<R, F><<<nb_site, kSiteThreads, 0, s>>>(c);
-    LAUNCHED(1);
-    scalar(op, 2);
+    launch(k_deriv<R, F>, fill(k_deriv<R, F>), kSiteThreads, 0, s, c, op);
   }
   static int set_smem_limits() {
     static bool done = false;
@@ -530,6 +555,10 @@ class Engine {
       v.sb[1] = c.sb[1];
       v.st = c.st;
       v.part = c.part;
+      v.tick = c.tick;
+      v.cst = c.cst;
+      v.csl = c.csl;
+      v.ctick = c.ctick;
       v.tw = c.tw;
       v.cs = c.cs;
       v.cs_ld = c.cs_ld;
@@ -548,39 +577,53 @@ class Engine {
   }
   void fft_xy(int bwd, int prsum) {
     const Ctx<F> v = cf();
-    if (xy_ct)
-      xy_ct<<<g_xy, bd_xy, sm_xy, s>>>(v, bwd, prsum);
-    else if (odd)
-      k_fft_xy<F, 16, true><<<g_xy, bd_xy, sm_xy, s>>>(v, bwd, prsum);
-    else if (pt_xy == 8)
-      k_fft_xy<F, 8, false><<<g_xy, bd_xy, sm_xy, s>>>(v, bwd, prsum);
-    else
-      k_fft_xy<F, 16, false><<<g_xy, bd_xy, sm_xy, s>>>(v, bwd, prsum);
-    LAUNCHED(1);
+    const XyFn<F> fn = xy_ct ? xy_ct
+                       : odd ? k_fft_xy<F, 16, true>
+                       : pt_xy == 8 ? k_fft_xy<F, 8, false> : k_fft_xy<F, 16, false>;
+    launch(fn, g_xy, bd_xy, sm_xy, s, v, bwd, prsum);
   }
   void fft_zt() {
     const Ctx<F> v = cf();
-    if (zt_ct)
-      zt_ct<<<g_zt, bd_zt, sm_zt, s>>>(v);
-    else if (odd)
-      k_fft_zt<F, 16, true><<<g_zt, bd_zt, sm_zt, s>>>(v);
-    else if (pt_zt == 8)
-      k_fft_zt<F, 8, false><<<g_zt, bd_zt, sm_zt, s>>>(v);
-    else
-      k_fft_zt<F, 16, false><<<g_zt, bd_zt, sm_zt, s>>>(v);
-    LAUNCHED(1);
+    const ZtFn<F> fn = zt_ct ? zt_ct
+                       : odd ? k_fft_zt<F, 16, true>
+                       : pt_zt == 8 ? k_fft_zt<F, 8, false> : k_fft_zt<F, 16, false>;
+    launch(fn, g_zt, bd_zt, sm_zt, s, v);
   }
   // direction + probes: FP64 storage one kernel; FP32 storage the FP32- and
   // the FP64-arithmetic variants, of which the device state picks one
   template <bool DIR>
-  void probe() {
+  void probe(int end) {
     if (sizeof(R) == 8) {
-      k_dir_probe<R, DIR, double, F><<<nb_site, kSiteThreads, 0, s>>>(c, SEL_ALWAYS);
+      probe_as<DIR, double>(SEL_ALWAYS, end);
     } else {
-      k_dir_probe<R, DIR, R, F><<<nb_site, kSiteThreads, 0, s>>>(c, SEL_LOW);
-      k_dir_probe<R, DIR, double, F><<<nb_site, kSiteThreads, 0, s>>>(c, SEL_HIGH);
-      LAUNCHED(1);
+      probe_as<DIR, R>(SEL_LOW, end);
+      probe_as<DIR, double>(SEL_HIGH, end);
     }
+  }
+  template <bool DIR, typename C>
+  void probe_as(int sel, int end) {
+    if constexpr (sizeof(C) == 8) {
+      if (!fuse_probes()) {
+        launch(k_dir_probe<R, DIR, C, F, false>, nb_site, kSiteThreads, 0, s, c, sel, end);
+        scalar(sel, OP_PROBES, end);
+        return;
+      }
+    }
+    const auto k = k_dir_probe<R, DIR, C, F, true>;
+    launch(k, fill(k), kSiteThreads, 0, s, c, sel, end);
+  }
+  // FP64 probes sum by tickets where a block for every 128 sites is one wave,
+  // else a scalar kernel follows
+  bool fuse_probes() {
+    return nb_site <= fill(k_dir_probe<R, true, double, F, false>, true);
+  }
+  void scalar(int sel, int op, int end) {
+    launch(k_scalar, 1, kScalarThreads, 0, s, d_st, (const double *)d_part, nb_site, sel, op,
+           end, (double)V);
+  }
+  template <bool SN>
+  void update() {
+    launch(k_update<R, SN, F>, nb_site, kSiteThreads, 0, s, c);
   }
   void fft(bool prsum) {
     fft_xy(0, 0);
@@ -592,28 +635,21 @@ class Engine {
   void sd_step(bool main, bool sd_fixed) {
     theta(main ? OP_THETA_MAIN : OP_THETA_SD);
     fft(false);
-    if (sd_fixed) {
-      scalar(OP_ALPHA_FIXED, 0);
-    } else {
-      probe<false>();
-      LAUNCHED(1);
-      scalar(OP_PROBES, 2);
-    }
-    k_update<R, false, F><<<nb_site, kSiteThreads, 0, s>>>(c);
-    LAUNCHED(1);
-    if (main) scalar(OP_END_SD, 0);
+    const int end = main ? OP_END_SD : OP_NONE;
+    if (!sd_fixed) probe<false>(end);
+    update<false>();
+    if (sd_fixed && main) scalar(SEL_ALWAYS, OP_NONE, end);
   }
   // one CG iteration (src/Gfix/FACG.c:270-334)
   void cg_iter() {
     theta(OP_THETA_MAIN);
     fft(true);
-    scalar(OP_PR, 2);
-    probe<true>();
-    LAUNCHED(1);
-    scalar(OP_PROBES, 2);
-    k_update<R, true, F><<<nb_site, kSiteThreads, 0, s>>>(c);
-    LAUNCHED(1);
-    scalar(OP_END_CG, 0);
+    probe<true>(OP_END_CG);
+    update<true>();
+  }
+  // sn = in_old = in after an SD start, and inold
+  void copy_der() {
+    launch(k_copy_der<F>, (V + 255) / 256, 256, 0, s, cf());
   }
 
   // Launch every kernel of the iteration once with the done flag set: each
@@ -625,7 +661,7 @@ class Engine {
     cg_iter();
     sd_step(true, false);
     sd_step(true, true);
-    k_copy_der<F><<<nb_site, kSiteThreads, 0, s>>>(cf());
+    copy_der();
     k_set_done<<<1, 1, 0, s>>>(d_st, 0);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
@@ -654,12 +690,13 @@ class Engine {
     return 0;
   }
 
-  unsigned long long per_iter_launches(bool cg, bool sd_fixed) const {
-    // k_deriv + scalar + 3 fft + ...
-    // (FP32 storage launches two probe variants)
+  unsigned long long per_iter_launches(bool cg, bool sd_fixed) {
+    // k_deriv, 3 FFT passes, the probes (FP32 storage launches two variants)
+    // and the update; a scalar step of its own on large lattices and for
+    // fixed SD steps
     const unsigned long long two = sizeof(R) == 4 ? 1 : 0;
-    if (cg) return 2 + 3 + 1 + 2 + 1 + 1 + two;
-    return 2 + 3 + (sd_fixed ? 1 : 2 + two) + 1 + 1;
+    if (!cg && sd_fixed) return 6;
+    return 6 + two + (fuse_probes() ? 0 : 1);
   }
 
   int read_state() {
@@ -788,9 +825,7 @@ class Engine {
     LAUNCHED(1);
     if (run_cg) {
       sd_step(false, run_p.sd_fixed != 0);
-      k_copy_der<F><<<nb_site, kSiteThreads, 0, s>>>(cf());
-      LAUNCHED(1);
-      scalar(OP_DER, 1);
+      copy_der();
     }
   }
 
@@ -869,54 +904,37 @@ class Engine {
   // events between the launches (no graph).  ms[k] = average duration of
   // one launch of kernel k, bytes[k] = its algorithmic HBM bytes:
   //   0 k_deriv, 1 k_fft_xy fwd, 2 k_fft_zt, 3 k_fft_xy bwd (+PR sums),
-  //   4 k_dir_probe, 5 k_update, 6 the four k_scalar launches together
+  //   4 k_dir_probe, 5 k_update, 6 nothing (the scalar steps go with the
+  //   kernels that sum)
   int profile_cg(const Params &p, int n, double *ms, double *bytes) {
     if (reset(p)) return -1;
     k_begin_run<<<1, 1, 0, s>>>(d_st);
     sd_step(false, p.sd_fixed != 0);
-    k_copy_der<F><<<nb_site, kSiteThreads, 0, s>>>(cf());
-    scalar(OP_DER, 1);
-    LAUNCHED(2);
+    copy_der();
+    LAUNCHED(1);
     std::vector<cudaEvent_t> ev(8);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
     for (int it = 0; it < n; it++) {
       CK(cudaEventRecord(ev[0], s));
-      k_deriv<R, F><<<nb_site, kSiteThreads, 0, s>>>(c);
+      theta(OP_THETA_MAIN);
       CK(cudaEventRecord(ev[1], s));
-      scalar(OP_THETA_MAIN, 2);
-      CK(cudaEventRecord(ev[2], s));
       fft_xy(0, 0);
-      CK(cudaEventRecord(ev[3], s));
-      fft_zt();
-      CK(cudaEventRecord(ev[4], s));
-      fft_xy(1, 1);
-      CK(cudaEventRecord(ev[5], s));
-      scalar(OP_PR, 2);
-      CK(cudaEventRecord(ev[6], s));
-      probe<true>();
-      CK(cudaEventRecord(ev[7], s));
-      CK(cudaStreamSynchronize(s));
-      float t[7];
-      for (int k = 0; k < 7; k++) CK(cudaEventElapsedTime(&t[k], ev[k], ev[k + 1]));
-      acc[0] += t[0];
-      acc[6] += t[1] + t[5];
-      acc[1] += t[2];
-      acc[2] += t[3];
-      acc[3] += t[4];
-      acc[4] += t[6];
-      CK(cudaEventRecord(ev[0], s));
-      scalar(OP_PROBES, 2);
-      CK(cudaEventRecord(ev[1], s));
-      k_update<R, true, F><<<nb_site, kSiteThreads, 0, s>>>(c);
       CK(cudaEventRecord(ev[2], s));
-      scalar(OP_END_CG, 0);
+      fft_zt();
       CK(cudaEventRecord(ev[3], s));
+      fft_xy(1, 1);
+      CK(cudaEventRecord(ev[4], s));
+      probe<true>(OP_END_CG);
+      CK(cudaEventRecord(ev[5], s));
+      update<true>();
+      CK(cudaEventRecord(ev[6], s));
       CK(cudaStreamSynchronize(s));
-      for (int k = 0; k < 3; k++) CK(cudaEventElapsedTime(&t[k], ev[k], ev[k + 1]));
-      acc[6] += t[0] + t[2];
-      acc[5] += t[1];
-      LAUNCHED(10);
+      float t;
+      for (int k = 0; k < 6; k++) {
+        CK(cudaEventElapsedTime(&t, ev[k], ev[k + 1]));
+        acc[k] += t;
+      }
     }
     for (auto &e : ev) cudaEventDestroy(e);
     // one complex number per site: of the links' type and of the fields'
@@ -958,13 +976,15 @@ class Engine {
     CK(cudaMallocHost(&h_sl, sizeof(Slice) * T));
     // per-slice partials: [T][nbs] pairs, next to the engine's own uses
     const size_t need = (size_t)T * nbs;
-    const size_t have =
-        std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y) + 1024;
+    const size_t have = std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y);
     if (need > have) {
       cudaFree(d_part);
-      CK(cudaMalloc(&d_part, (need + 1024) * 2 * sizeof(double)));
+      d_part = nullptr;
+      CK(cudaMalloc(&d_part, (need + tick_groups((unsigned)need)) * 2 * sizeof(double)));
       c.part = d_part;
     }
+    c.cst = d_cst;
+    c.csl = d_sl;
     cc.U = d_U;
     cc.g = d_G;
     cc.fb[0] = c.fb[0];
@@ -975,18 +995,12 @@ class Engine {
     cc.cs = d_cst;
     cc.sl = d_sl;
     cc.part = d_part;
+    cc.tick = c.ctick;
     for (int i = 0; i < 4; i++) cc.L[i] = c.L[i];
     cc.V = V;
     cc.Lcu = Lcu;
     cc.nbs = nbs;
     return 0;
-  }
-
-  void cscalar(int op) {
-    const int T = c.L[3];
-    k_cscalar<<<(T + kCScalarSlices - 1) / kCScalarSlices, 32 * kCScalarSlices, 0, s>>>(
-        d_cst, d_sl, d_part, nbs, c.L[2], c.L[2] * T, op, (double)Lcu, d_st);
-    LAUNCHED(1);
   }
 
   void capture_coul() {
@@ -1012,21 +1026,32 @@ class Engine {
   // FP32- and an FP64-arithmetic variant, each taking its own slices
   void cderiv(dim3 gs) {
     if (sizeof(R) == 8) {
-      k_cderiv<R, double><<<gs, kCoulThreads, 0, s>>>(cc, SEL_ALWAYS);
+      launch(k_cderiv<R, double>, gs, kCoulThreads, 0, s, cc, SEL_ALWAYS);
     } else {
-      k_cderiv<R, R><<<gs, kCoulThreads, 0, s>>>(cc, SEL_LOW);
-      k_cderiv<R, double><<<gs, kCoulThreads, 0, s>>>(cc, SEL_HIGH);
-      LAUNCHED(1);
+      launch(k_cderiv<R, R>, gs, kCoulThreads, 0, s, cc, SEL_LOW);
+      launch(k_cderiv<R, double>, gs, kCoulThreads, 0, s, cc, SEL_HIGH);
     }
   }
   void cprobe(dim3 gs) {
     if (sizeof(R) == 8) {
-      k_cprobe<R, double><<<gs, kCoulThreads, 0, s>>>(cc, SEL_ALWAYS);
+      launch(k_cprobe<R, double>, gs, kCoulThreads, 0, s, cc, SEL_ALWAYS);
     } else {
-      k_cprobe<R, R><<<gs, kCoulThreads, 0, s>>>(cc, SEL_LOW);
-      k_cprobe<R, double><<<gs, kCoulThreads, 0, s>>>(cc, SEL_HIGH);
-      LAUNCHED(1);
+      launch(k_cprobe<R, R>, gs, kCoulThreads, 0, s, cc, SEL_LOW);
+      launch(k_cprobe<R, double>, gs, kCoulThreads, 0, s, cc, SEL_HIGH);
     }
+  }
+  void cscalar(int op) {
+    const int T = c.L[3];
+    launch(k_cscalar, (T + kCScalarSlices - 1) / kCScalarSlices, 32 * kCScalarSlices, 0, s,
+           d_cst, d_sl, (const double *)d_part, nbs, (int)g_xy.x / T, op, (double)Lcu, d_st);
+  }
+  void cupdate(dim3 gs) {
+    launch(k_cupdate<R>, gs, kCoulThreads, 0, s, cc);
+  }
+  void cmaint() {
+    const dim3 gm(std::min(nbs, kMaintBlocks), c.L[3]);
+    launch(k_cmaint<R>, gm, kCoulThreads, 0, s, cc, 0);
+    launch(k_cmaint<R>, gm, kCoulThreads, 0, s, cc, 1);
   }
 
   // one step of every live slice
@@ -1035,17 +1060,12 @@ class Engine {
     cderiv(gs);
     fft_xy(0, 0);
     fft_zt();
-    fft_xy(1, 1);  // with the per-plane sums of the accelerated field
+    fft_xy(1, 1);  // with the partials of the accelerated field's sums
     cscalar(C_SUMS);
     cprobe(gs);
     cscalar(C_PROBES);
-    k_cupdate<R><<<gs, kCoulThreads, 0, s>>>(cc);
-    cscalar(C_END1);
-    k_cmaint<R><<<gs, kCoulThreads, 0, s>>>(cc, 0);
-    cscalar(C_END2);
-    k_cmaint<R><<<gs, kCoulThreads, 0, s>>>(cc, 1);
-    k_cflip<<<1, 1, 0, s>>>(d_st);
-    LAUNCHED(6);
+    cupdate(gs);
+    cmaint();
   }
 
   // GLU's Coulomb_FA (src/Gfix/CFACG.c:531-636) on the resident links
@@ -1115,7 +1135,7 @@ class Engine {
     const int T = c.L[3];
     const size_t per = p.traj_cap ? p.traj_cap / T : 0;
     // launches in citer() (FP32 storage: two variants of two kernels)
-    const unsigned long long per_iter = sizeof(R) == 4 ? 15 : 13;
+    const unsigned long long per_iter = sizeof(R) == 4 ? 12 : 10;
     int batch = 2;
     size_t guard = 0;
     const size_t limit = (p.max_iters + 2) * 9 * 64 + 1024;
@@ -1172,8 +1192,8 @@ class Engine {
   // Measurement aid: n steps of every slice (none may finish: accuracy 0)
   // with CUDA events between the launches; ms[k] = mean time of launch k:
   // 0 derivative, 1 xy FFT forward, 2 z FFT with psq, 3 xy FFT inverse +
-  // sums, 4 direction + probes, 5 g update, 6 the scalar, housekeeping and
-  // parity launches of a step; bytes[k] = its algorithmic HBM bytes.
+  // sums, 4 direction + probes, 5 g update, 6 the scalar and housekeeping
+  // launches of a step; bytes[k] = its algorithmic HBM bytes.
   int profile_coul(const Params &p, int n, double *ms, double *bytes) {
     Params q = p;
     q.acc = 0.0;
@@ -1200,22 +1220,14 @@ class Engine {
       CK(cudaEventRecord(ev[6], s));
       cscalar(C_PROBES);
       CK(cudaEventRecord(ev[7], s));
-      k_cupdate<R><<<gs, kCoulThreads, 0, s>>>(cc);
+      cupdate(gs);
       CK(cudaEventRecord(ev[8], s));
-      cscalar(C_END1);
-      k_cmaint<R><<<gs, kCoulThreads, 0, s>>>(cc, 0);
-      cscalar(C_END2);
-      k_cmaint<R><<<gs, kCoulThreads, 0, s>>>(cc, 1);
-      k_cflip<<<1, 1, 0, s>>>(d_st);
+      cmaint();
       CK(cudaEventRecord(ev[9], s));
-      LAUNCHED(6);
       CK(cudaStreamSynchronize(s));
       float t[9];
       for (int k = 0; k < 9; k++) CK(cudaEventElapsedTime(&t[k], ev[k], ev[k + 1]));
-      acc[0] += t[0];
-      acc[1] += t[1];
-      acc[2] += t[2];
-      acc[3] += t[3];
+      for (int k = 0; k < 4; k++) acc[k] += t[k];
       acc[4] += t[5];
       acc[5] += t[7];
       acc[6] += t[4] + t[6] + t[8];

@@ -1,17 +1,18 @@
 // Device kernels of the Fourier-accelerated Landau gauge fixing on B200.
 //
 // One iteration of FACG (src/Gfix/FACG.c:270-334) is the launch sequence
-//   k_deriv          Delta(x) packed in 4 fields + theta and Re tr U partials
-//   k_scalar THETA   theta, functional, stop decision
+//   k_deriv          Delta(x) packed in 4 fields, then theta, functional and
+//                    the stop decision
 //   k_fft_xy  fwd    x,y passes of the 4D FFT, one xy-plane per block
 //   k_fft_zt         z,t passes, * psq, inverse t,z passes (one tile/block)
-//   k_fft_xy  bwd    inverse x,y passes fused with the PR sums
-//   k_scalar PR      beta (PR+ / FR switch at CG_TOL)
+//   k_fft_xy  bwd    inverse x,y passes fused with the PR sums, then beta
+//                    (PR+ / FR switch at CG_TOL)
 //   k_dir_probe      sn <- in + beta sn, line-search probes of GLU's
-//                    line_search_Landau (src/Gfix/line_search.c:274-341)
-//   k_scalar PROBES  alpha* by the parabola of approx_minimum
-//   k_update         U_mu(x) <- g(x) U_mu(x) g(x+mu)^dag, g = reunit(1+a A)
-//   k_scalar END     iteration count, buffer parities, done flag
+//                    line_search_Landau (src/Gfix/line_search.c:274-341), then
+//                    alpha* by the parabola of approx_minimum
+//   k_update         U_mu(x) <- g(x) U_mu(x) g(x+mu)^dag, g = reunit(1+a A),
+//                    then iteration count, buffer parities, done flag
+// The scalar steps are taken by the last block of each kernel (control.cuh).
 // Every kernel first checks the device-side done flag, so a captured graph
 // of the iteration can be replayed past convergence as a no-op.
 //
@@ -28,70 +29,16 @@
 // carries its search directions and their Fourier acceleration in FP32.
 #pragma once
 
+#include "control.cuh"
 #include "fft.cuh"
-#include "su3.cuh"
 
 namespace gfix {
 
-constexpr double kCgTol = 5E-11;            // GLU_definitions.h:451-455
-constexpr double kVal49 = 0.4444444444444444;  // lin_derivs.c:72
-constexpr int kSiteThreads = 128;
-constexpr int kScalarThreads = 1024;
-
-enum ScalarOp : int {
-  OP_THETA_TEST = 0,  // theta_test_lin = 2 sum / (NC V)
-  OP_THETA_SD,        // theta of an SD start: reduction slots carry over
-  OP_THETA_MAIN,      // theta at the top of a CG/SD iteration
-  OP_PR,              // beta of the CG direction
-  OP_PROBES,          // alpha* from the probes (or the fixed step)
-  OP_DER,             // inold after the SD start
-  OP_END_CG,          // end of a CG iteration
-  OP_END_SD,          // end of an SD (FASD) iteration
-  OP_ALPHA_FIXED,     // step = gf_alpha (SD without line search)
-};
-
-struct DevState {
-  double tr;          // in-loop theta of the current iteration
-  double tr_test;     // theta_test_lin
-  double func;        // gauge functional of the current links
-  double inold, insum, sumconj, beta, alpha;
-  double ls_last[2];  // probe sums left in GLU's reduction slots
-  double insum_last;  // insum left in GLU's reduction slot
-  double gf_alpha, acc;
-  long long max_iters;
-  long long iter;     // loc_iters of the current run
-  long long traj_len, traj_cap;
-  double *traj_theta, *traj_func;
-  int use_ls;         // this step uses the line search
-  int stop;           // current iteration is the last one of the run
-  int done;           // run finished: kernels return at once
-  int parity;         // fb[parity] = in, fb[parity ^ 1] = in_old
-  int sparity;        // sb[sparity] = sn (old), sb[sparity ^ 1] = new
-  int nblocks;        // partials written by the last reduction kernel
-  int sd_fixed;       // GLU_GFIX_SD: fixed step gf_alpha in SD steps
-  double cg_tol;      // CG_TOL (GLU_definitions.h:451-455)
-  double hp_below;    // FP32 storage: probes in FP64 arithmetic once tr < this
-  // stall rule of a mixed-precision FP32 phase (stall_window 0: off): once
-  // the best theta is below stall_floor, the run ends when theta has not
-  // improved on it by 10% for stall_window iterations or exceeds blowup x it
-  double best_tr, stall_floor, blowup;
-  long long since_best, stall_window;
-};
-
-// which arithmetic variant of a kernel runs this step (FP32 storage: FP32
-// arithmetic while theta >= hp_below, FP64 arithmetic below; a NaN theta
-// takes the FP32 variant)
-enum ArithSel : int { SEL_ALWAYS = 0, SEL_LOW = 1, SEL_HIGH = 2 };
-__device__ __forceinline__ bool arith_skip(int sel, double tr, double below) {
-  const bool high = tr < below;
-  return (sel == SEL_LOW && high) || (sel == SEL_HIGH && !high);
-}
-
 // set or clear the done flag (used to run every kernel once as a no-op)
-__global__ void k_set_done(DevState *st, int v) { st->done = v; }
+static __global__ void k_set_done(DevState *st, int v) { st->done = v; }
 
 // start of a solver run (GLU's steep_Landau_FACG / _FASD entry)
-__global__ void k_begin_run(DevState *st) {
+static __global__ void k_begin_run(DevState *st) {
   st->iter = 0;
   st->done = 0;
   st->stop = 0;
@@ -105,7 +52,8 @@ struct Ctx {
   cx<F> *sb[2];
   cx<R> *G;
   DevState *st;
-  double *part;       // [nblocks][2] per-block partial sums
+  double *part;       // [nblocks][2] per-block partial sums, group totals
+  unsigned *tick;     // tickets of grid_sum, zero between kernels
   const cx<F> *tw;    // twiddle pool
   const double *cs;   // cos tables, cs[mu * cs_ld + n] = cos(n 2pi/L_mu)
   int cs_ld;
@@ -117,39 +65,13 @@ struct Ctx {
   double maxp;        // MAX_LANDAU = 4 ND / V or MAX_COULOMB = 4 (ND-1)/Lcu
   FftAxis ax[4];
   const int *skip;    // ndim 3: per-slice flags, set slices are not transformed
+  CoulState *cst;     // ndim 3: control of the slices, and a ticket for each
+  Slice *csl;
+  unsigned *ctick;
 };
 
 // ---------------------------------------------------------------------
 // helpers
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// deterministic block sum of NV values; thread 0 writes them to out[0..NV)
-template <int NV>
-__device__ __forceinline__ void block_sum_store(double (&v)[NV], double *out) {
-  __shared__ double sh[NV][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; k++) v[k] = warp_sum(v[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; k++) sh[k][warp] = v[k];
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      double x = lane < nw ? sh[k][lane] : 0.0;
-      x = warp_sum(x);
-      if (lane == 0) out[k] = x;
-    }
-  }
-}
 
 // buffer of a ping-pong pair by parity, as a select (a runtime index into
 // the by-value kernel parameter would copy it to local memory)
@@ -244,12 +166,11 @@ __device__ __forceinline__ void store_link(cx<R> *U, int V, int mu, int s,
 // (src/Gfix/lin_derivs.c:74-193 packed as src/Gfix/FACG.c:54-60)
 
 template <typename R, typename F = R>
-__global__ void __launch_bounds__(kSiteThreads)
-    k_deriv(Ctx<R, F> c) {
+__global__ void __launch_bounds__(kSiteThreads, sizeof(R) == 8 ? 5 : 7)
+    k_deriv(Ctx<R, F> c, int op) {
   if (c.st->done) return;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
   double v[2] = {0.0, 0.0};
-  if (s < c.V) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < c.V; s += gridDim.x * blockDim.x) {
     int x[4], sd[4];
     coords(s, c.L, x);
     strides(c, sd);
@@ -284,12 +205,13 @@ __global__ void __launch_bounds__(kSiteThreads)
     f[3 * V + s] = mk<F>((F)(R(0.5) * R4), (F)(R(0.5) * I4));
     const double d0 = R0, d1 = R1, e1 = I1, d2 = R2, e2 = I2, d3 = R3,
                  d4 = R4, e4 = I4;
-    v[0] = kVal49 * (d0 * d0 + d3 * (d3 + d0)) +
+    v[0] += kVal49 * (d0 * d0 + d3 * (d3 + d0)) +
            (d1 * d1 + e1 * e1 + d2 * d2 + e2 * e2 + d4 * d4 + e4 * e4);
-    v[1] = re;
+    v[1] += re;
   }
-  block_sum_store<2>(v, c.part + 2 * blockIdx.x);
-  if (threadIdx.x == 0 && blockIdx.x == 0) c.st->nblocks = gridDim.x;
+  grid_sum_begin(v, c.part, c.tick, blockIdx.x, gridDim.x);
+  if (grid_sum(v, c.part, c.tick, blockIdx.x, gridDim.x))
+    apply_scalar(c.st, op, v[0], v[1], (double)c.V);
 }
 
 // ---------------------------------------------------------------------
@@ -342,8 +264,8 @@ __device__ __forceinline__ void dir_at(const Ctx<R, F> &c, const cx<F> *in,
 // 0.23 ms in FP32.  Blocks per SM: four (128 registers) in FP64, three take
 // 0.393 ms; six in FP32, four 0.237 ms.  Both probes unrolled together spill
 // (0.685 ms).
-template <typename R, bool DIR, typename C = R, typename F = R>
-__global__ void __launch_bounds__(kSiteThreads, sizeof(C) == 4 ? 6 : 4) k_dir_probe(Ctx<R, F> c, int sel) {
+template <typename R, bool DIR, typename C, typename F, bool FUSED>
+__global__ void __launch_bounds__(kSiteThreads, sizeof(C) == 4 ? 6 : 4) k_dir_probe(Ctx<R, F> c, int sel, int end) {
   if (c.st->done || arith_skip(sel, c.st->tr, c.st->hp_below)) return;
   __shared__ cx<C> sA[2][9][kSiteThreads];  // g(x) at both probes
   const int par = c.st->parity, spar = c.st->sparity;
@@ -352,9 +274,9 @@ __global__ void __launch_bounds__(kSiteThreads, sizeof(C) == 4 ? 6 : 4) k_dir_pr
   cx<F> *sn = pick(c.sb, spar ^ 1);
   const R beta = (R)c.st->beta;
   const bool probes = c.st->use_ls != 0;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
   double v[2] = {0.0, 0.0};
-  if (s < c.V) {
+  const int s0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int s = s0; s < c.V; s += gridDim.x * blockDim.x) {
     cx<R> f[4];
     cx<F> fs[4];
     dir_at<R, DIR>(c, in, so, beta, s, f, fs);
@@ -394,28 +316,73 @@ __global__ void __launch_bounds__(kSiteThreads, sizeof(C) == 4 ? 6 : 4) k_dir_pr
           d[k] += probe_trace(A, w0, w1, p, k == 0 ? C(0.15) : C(0.30)) - t0;
         }
       }
-      v[0] = d[0];
-      v[1] = d[1];
+      v[0] += d[0];
+      v[1] += d[1];
     }
+    if (!FUSED) break;
   }
-  if (probes) {
-    block_sum_store<2>(v, c.part + 2 * blockIdx.x);
-    if (threadIdx.x == 0 && blockIdx.x == 0) c.st->nblocks = gridDim.x;
+  if constexpr (!FUSED) {
+    if (probes) block_sum_store<2>(v, c.part + 2 * blockIdx.x);
+    return;
+  }
+  grid_sum_begin(v, c.part, c.tick, blockIdx.x, gridDim.x);
+  if (grid_sum(v, c.part, c.tick, blockIdx.x, gridDim.x)) {
+    apply_scalar(c.st, OP_PROBES, v[0], v[1], (double)c.V);
+    apply_scalar(c.st, end, 0.0, 0.0, (double)c.V);
   }
 }
+
+// the probes' scalar step by a kernel of its own, where their grid has a block
+// for every 128 sites of a large lattice and a ticket for each would cost
+// more; sel: of the probes' variant.  op: OP_PROBES with `end`, or OP_NONE with
+// `end` alone
+constexpr int kScalarThreads = 1024;
+static __global__ void __launch_bounds__(kScalarThreads)
+    k_scalar(DevState *st, const double *part, int nb, int sel, int op, int end, double V) {
+  if (st->done || arith_skip(sel, st->tr, st->hp_below)) return;
+  double v[2] = {0.0, 0.0};
+  if (op != OP_NONE) {
+    // eight independent loads in flight per thread and round, then added in a
+    // fixed order
+    constexpr int kU = 8;
+    const double2 *p = reinterpret_cast<const double2 *>(part);
+    for (int i0 = threadIdx.x; i0 < nb; i0 += kU * kScalarThreads) {
+      double2 x[kU];
+#pragma unroll
+      for (int k = 0; k < kU; k++) {
+        const int i = i0 + k * kScalarThreads;
+        x[k] = i < nb ? p[i] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int k = 0; k < kU; k++) {
+        v[0] += x[k].x;
+        v[1] += x[k].y;
+      }
+    }
+    __shared__ double tot[2];
+    block_sum_store<2>(v, tot);
+    v[0] = tot[0];
+    v[1] = tot[1];
+  }
+  if (threadIdx.x != 0) return;
+  apply_scalar(st, op, v[0], v[1], V);
+  apply_scalar(st, end, 0.0, 0.0, V);
+}
+
 
 // ---------------------------------------------------------------------
 // K5: the link update of egauge_Landau (src/Gfix/line_search.c:60-97):
 // g(x) = reunit(1 + alpha A(x)), U_mu(x) <- g(x) U_mu(x) g(x+mu)^dag.
-// SN selects the direction: the new conjugate direction or `in`.
+// SN selects the direction: the new conjugate direction or `in` (the end of
+// the iteration, which flips sn's buffers, has been applied with the probes').
 // With G (mixed precision) the transform is accumulated, G(x) <- g(x) G(x).
 
 template <typename R, bool SN, typename F = R>
 __global__ void __launch_bounds__(kSiteThreads) k_update(Ctx<R, F> c) {
-  if (c.st->done) return;
+  if (!c.st->upd) return;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= c.V) return;
-  const cx<F> *d = SN ? c.sb[c.st->sparity ^ 1] : c.fb[c.st->parity];
+  const cx<F> *d = SN ? c.sb[c.st->sparity] : c.fb[c.st->parity];
   const R alpha = (R)c.st->alpha;
   const size_t V = c.V;
   int x[4], sd[4];
@@ -449,7 +416,7 @@ __global__ void __launch_bounds__(256) k_copy_der(Ctx<R> c) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const cx<R> *in = c.fb[c.st->parity];
   cx<R> *sn = c.sb[c.st->sparity];
-  double v[1] = {0.0};
+  double v[2] = {0.0, 0.0};
   if (s < c.V) {
     double l = 0.0;
 #pragma unroll
@@ -461,136 +428,9 @@ __global__ void __launch_bounds__(256) k_copy_der(Ctx<R> c) {
     }
     v[0] = 2.0 * l;
   }
-  block_sum_store<1>(v, c.part + blockIdx.x);
-  if (threadIdx.x == 0 && blockIdx.x == 0) c.st->nblocks = gridDim.x;
-}
-
-// ---------------------------------------------------------------------
-// scalar logic: one block reduces the partials in a fixed order and applies
-// GLU's control flow for the step.
-
-__device__ __forceinline__ double approx_minimum(const double *al,
-                                                 const double *f) {
-  // src/Gfix/line_search.c:38-57
-  const double A = f[0] / ((al[0] - al[1]) * (al[0] - al[2]));
-  const double B = f[1] / ((al[1] - al[0]) * (al[1] - al[2]));
-  const double C = f[2] / ((al[2] - al[0]) * (al[2] - al[1]));
-  const double Sol = (al[0] * (B + C) + al[1] * (A + C) + al[2] * (A + B)) /
-                     (2 * (A + B + C));
-  if (Sol > al[2]) return al[2];
-  if (isnan(Sol) || isinf(Sol) || Sol < al[0]) return 0.08;
-  return Sol;
-}
-
-__global__ void __launch_bounds__(kScalarThreads)
-    k_scalar(DevState *st, const double *part, int op, int nv, double norm_v) {
-  if (st->done) return;
-  const int nb = st->nblocks;
-  double a[2] = {0.0, 0.0};
-  if (op != OP_END_CG && op != OP_END_SD && op != OP_ALPHA_FIXED) {
-    // eight independent loads in flight per thread and round, then added
-    // in a fixed order: the sum is deterministic and pays the L2 latency
-    // once per eight partials instead of once per partial
-    constexpr int kU = 8;
-    const int B = blockDim.x;
-    for (int i0 = threadIdx.x; i0 < nb; i0 += kU * B) {
-      double x0[kU], x1[kU];
-#pragma unroll
-      for (int k = 0; k < kU; k++) {
-        const int i = i0 + k * B;
-        x0[k] = i < nb ? part[(size_t)nv * i] : 0.0;
-        x1[k] = (nv > 1 && i < nb) ? part[(size_t)nv * i + 1] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < kU; k++) {
-        a[0] += x0[k];
-        a[1] += x1[k];
-      }
-    }
-    __shared__ double tot[2];
-    block_sum_store<2>(a, tot);
-    __syncthreads();
-    a[0] = tot[0];
-    a[1] = tot[1];
-  }
-  if (threadIdx.x != 0) return;
-  // norm_v = number of sites V
-  const double V = norm_v;
-  switch (op) {
-    case OP_THETA_TEST:
-      st->tr_test = 2.0 * a[0] / (3.0 * V);
-      st->func = 1.0 - a[1] / (12.0 * V);
-      break;
-    case OP_THETA_SD:
-    case OP_THETA_MAIN: {
-      st->tr = a[0] / (3.0 * V);  // GFNORM_LANDAU
-      st->func = 1.0 - a[1] / (12.0 * V);
-      if (st->traj_theta && st->traj_len < st->traj_cap) {
-        st->traj_theta[st->traj_len] = st->tr;
-        st->traj_func[st->traj_len] = st->func;
-        st->traj_len++;
-      }
-      if (op == OP_THETA_MAIN) {
-        // the top of a loop iteration zeroes GLU's reduction slots
-        st->ls_last[0] = st->ls_last[1] = 0.0;
-        st->stop = !((st->tr > st->acc) && (st->iter + 1 < st->max_iters));
-        if (st->stall_window > 0) {
-          if (st->tr < 0.9 * st->best_tr) {
-            st->best_tr = st->tr;
-            st->since_best = 0;
-          } else {
-            st->since_best++;
-          }
-          if (st->best_tr < st->stall_floor &&
-              (st->since_best >= st->stall_window || st->tr > st->blowup * st->best_tr))
-            st->stop = 1;
-        }
-      }
-      break;
-    }
-    case OP_PR: {
-      st->insum = a[0];
-      st->sumconj = a[1];
-      const double b = st->sumconj / st->inold;
-      double beta = (b < 0.0) ? 0.0 : b;  // PRfmax (src/Gfix/CG.c:37-41)
-      if (st->tr < st->cg_tol) beta = st->insum / st->inold;
-      st->beta = beta;
-      st->inold = st->insum;
-      st->insum_last = st->insum;
-      st->use_ls = st->tr > st->cg_tol;
-      break;
-    }
-    case OP_PROBES: {
-      if (st->use_ls) {
-        const double d1 = a[0] + st->ls_last[0], d2 = a[1] + st->ls_last[1];
-        st->ls_last[0] = d1;
-        st->ls_last[1] = d2;
-        const double al[3] = {0.0, 0.15, 0.30};
-        const double f[3] = {0.0, -d1, -d2};
-        st->alpha = approx_minimum(al, f);
-      } else {
-        st->alpha = st->gf_alpha;
-      }
-      break;
-    }
-    case OP_ALPHA_FIXED:
-      st->alpha = st->gf_alpha;
-      break;
-    case OP_DER:
-      st->inold = st->insum_last + a[0];
-      st->parity ^= 1;  // in_old = in
-      break;
-    case OP_END_CG:
-      st->iter++;
-      st->parity ^= 1;
-      st->sparity ^= 1;
-      if (st->stop) st->done = 1;
-      break;
-    case OP_END_SD:
-      st->iter++;
-      if (st->stop) st->done = 1;
-      break;
-  }
+  grid_sum_begin(v, c.part, c.tick, blockIdx.x, gridDim.x);
+  if (grid_sum(v, c.part, c.tick, blockIdx.x, gridDim.x))
+    apply_scalar(c.st, OP_DER, v[0], v[1], (double)c.V);
 }
 
 // ---------------------------------------------------------------------

@@ -304,7 +304,8 @@ int gfix_fourier_accelerate(double *fields, const size_t dims[4], int ndim);
  * ms[k] = mean duration of one launch of kernel k, bytes[k] = algorithmic
  * HBM bytes of one launch, for k = 0 derivative+theta, 1 xy FFT forward,
  * 2 zt FFT with psq, 3 xy FFT inverse + PR sums, 4 direction + line-search
- * probes, 5 link update, 6 the scalar-control launches of one iteration.
+ * probes (with their scalar step), 5 link update, 6 nothing (zero: the scalar
+ * steps go with the kernels that sum).
  * precision GFIX_MIXED profiles the FP32 kernels, GFIX_PROFILE_POLISH those
  * of a mixed solve's FP64-link phase. */
 int gfix_profile_landau(const double *d_links, const size_t dims[4],
@@ -316,8 +317,8 @@ int gfix_profile_landau(const double *d_links, const size_t dims[4],
  * with CUDA events between the launches.  ms[k] / bytes[k] as for
  * gfix_profile_landau, for k = 0 derivative, 1 xy FFT forward, 2 z FFT with
  * psq, 3 xy FFT inverse + the per-slice sums, 4 direction + line-search
- * probes, 5 update of the slice gauge fields, 6 the scalar, housekeeping and
- * parity launches of one step.  precision GFIX_MIXED profiles the FP32
+ * probes, 5 update of the slice gauge fields, 6 the scalar and housekeeping
+ * launches of one step.  precision GFIX_MIXED profiles the FP32
  * kernels. */
 int gfix_profile_coulomb(const double *d_links, const size_t dims[4],
                          const gfix_params *p, int iters, double *ms,
