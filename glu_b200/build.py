@@ -18,8 +18,10 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libglu_gfix.so"
-SOURCES = ["gfix.cu", "glu_abi.cu", "noalloc.cu", "nersc.cu", "cuts.cu", "update.cu"]
-HEADERS = ["su3.cuh", "control.cuh", "fft.cuh", "fft_pass.cuh", "fft_ct.cuh", "kernels.cuh", "extra_kernels.cuh",
+SOURCES = ["gfix.cu", "glu_abi.cu", "noalloc.cu", "nersc.cu", "cuts.cu", "update.cu",
+           "fft_xy_f32.cu", "fft_xy_f64.cu", "fft_zt_f32.cu", "fft_zt_f64.cu"]
+HEADERS = ["su3.cuh", "control.cuh", "fft.cuh", "fft_pass.cuh", "fft_ct.cuh", "fft_reg.cuh", "fft_reg_api.cuh",
+           "kernels.cuh", "extra_kernels.cuh",
            "coulomb.cuh", "glu_compat.h", "su3_log.cuh", "drop_in.h"]
 
 NVCC_FLAGS = [

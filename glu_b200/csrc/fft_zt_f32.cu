@@ -1,0 +1,47 @@
+// Register-pencil (z, t) and Coulomb z passes, float (fft_reg.cuh)
+#include "fft_reg.cuh"
+#include "fft_reg_api.cuh"
+
+namespace gfix {
+
+template <>
+RegZt<float> reg_zt<float>(int lz, int lt, int lx, int want) {
+  RegZt<float> r;
+#define GFIX_T(LZ, LT, B) GFIX_TW(LZ, LT, B, B)
+#define GFIX_TW(LZ, LT, B, W)                                                       \
+  if (lz == LZ && lt == LT && lx % B == 0 && (want ? want == B : !r.fn)) {          \
+    r.fn = k_fft_zt_reg<float, LZ, LT, B, W>;                                       \
+    r.columns = B;                                                                  \
+    r.threads = zt_reg_threads<float, LZ, LT, W>();                                \
+    r.smem = zt_reg_smem<float, LZ, LT, W>();                                      \
+  }
+  GFIX_T(4, 4, 4) GFIX_T(4, 8, 4) GFIX_T(8, 8, 4) GFIX_T(8, 16, 4) GFIX_T(12, 12, 4)
+  GFIX_T(12, 24, 4) GFIX_T(16, 16, 4) GFIX_T(16, 32, 4) GFIX_T(20, 20, 4) GFIX_T(20, 40, 4)
+  GFIX_T(24, 24, 4) GFIX_T(24, 48, 4) GFIX_T(4, 4, 2) GFIX_T(4, 8, 2) GFIX_T(8, 8, 2)
+  GFIX_T(8, 16, 2) GFIX_T(16, 16, 2) GFIX_T(16, 32, 2) GFIX_T(24, 48, 2) GFIX_T(32, 32, 2)
+  GFIX_T(28, 28, 4) GFIX_T(32, 32, 4)
+  GFIX_T(6, 6, 2) GFIX_T(6, 12, 2) GFIX_T(10, 10, 2) GFIX_T(10, 20, 2) GFIX_T(14, 14, 2)
+  GFIX_T(14, 28, 2) GFIX_T(18, 18, 2) GFIX_T(30, 30, 2)
+  GFIX_T(28, 56, 4) GFIX_T(32, 64, 4) GFIX_T(32, 64, 2) GFIX_T(32, 64, 1)
+  GFIX_T(18, 36, 2) GFIX_T(30, 60, 2) GFIX_T(36, 36, 2) GFIX_T(36, 72, 2) GFIX_T(40, 40, 2)
+  GFIX_T(40, 80, 2) GFIX_T(48, 48, 2) GFIX_T(48, 96, 2) GFIX_T(48, 96, 1)
+#undef GFIX_T
+#undef GFIX_TW
+  return r;
+}
+
+template <>
+RegZt<float> reg_z<float>(int lz) {
+  RegZt<float> r;
+#define GFIX_Z(N)                    \
+  if (lz == N) {                     \
+    r.fn = k_fft_z_reg<float, N>;   \
+    r.threads = kZThreads;           \
+  }
+  GFIX_Z(4) GFIX_Z(6) GFIX_Z(8) GFIX_Z(10) GFIX_Z(12) GFIX_Z(14) GFIX_Z(16) GFIX_Z(18)
+  GFIX_Z(20) GFIX_Z(24) GFIX_Z(28) GFIX_Z(30) GFIX_Z(32) GFIX_Z(36) GFIX_Z(40) GFIX_Z(48)
+#undef GFIX_Z
+  return r;
+}
+
+}  // namespace gfix

@@ -27,6 +27,7 @@
 #include "coulomb.cuh"
 #include "drop_in.h"
 #include "extra_kernels.cuh"
+#include "fft_reg_api.cuh"
 #include "kernels.cuh"
 
 namespace gfix {
@@ -86,13 +87,14 @@ using XyFn = void (*)(Ctx<R>, int, int);
 template <typename R>
 using ZtFn = void (*)(Ctx<R>);
 
+// (the extents whose register-pencil passes would need more registers than a
+// thread has: fft_reg_api.cuh)
 template <typename R>
 static XyFn<R> ct_xy(int lx, int ly) {
-#define GFIX_XY(n) \
-  if (lx == n && ly == n) return k_fft_xy_ct<R, n, n>;
-  GFIX_XY(4) GFIX_XY(8) GFIX_XY(16) GFIX_XY(24) GFIX_XY(32) GFIX_XY(48)
-  GFIX_XY(64)
-#undef GFIX_XY
+  if constexpr (sizeof(R) == 8) {
+    if (lx == 48 && ly == 48) return k_fft_xy_ct<R, 48, 48>;
+    if (lx == 64 && ly == 64) return k_fft_xy_ct<R, 64, 64>;
+  }
   return nullptr;
 }
 
@@ -100,14 +102,11 @@ template <typename R>
 static ZtFn<R> ct_zt(int lz, int lt, int b) {
 #define GFIX_ZT(z, t, bb) \
   if (lz == z && lt == t && b == bb) return k_fft_zt_ct<R, z, t, bb>;
-  GFIX_ZT(4, 4, 2) GFIX_ZT(4, 8, 2) GFIX_ZT(8, 8, 2) GFIX_ZT(8, 16, 2)
-  GFIX_ZT(16, 16, 2) GFIX_ZT(16, 32, 2) GFIX_ZT(24, 48, 2)
-  GFIX_ZT(32, 32, 2) GFIX_ZT(32, 64, 2) GFIX_ZT(48, 96, 2)
-  GFIX_ZT(32, 64, 1) GFIX_ZT(32, 64, 4) GFIX_ZT(48, 96, 1) GFIX_ZT(16, 32, 4)
-  GFIX_ZT(4, 1, 8) GFIX_ZT(8, 1, 8) GFIX_ZT(16, 1, 8) GFIX_ZT(24, 1, 8)
-  GFIX_ZT(32, 1, 8) GFIX_ZT(48, 1, 8) GFIX_ZT(64, 1, 8)
-  GFIX_ZT(8, 1, 16) GFIX_ZT(16, 1, 16) GFIX_ZT(24, 1, 16) GFIX_ZT(32, 1, 16)
-  GFIX_ZT(48, 1, 16) GFIX_ZT(64, 1, 16) GFIX_ZT(32, 1, 32) GFIX_ZT(64, 1, 32)
+  GFIX_ZT(64, 1, 8) GFIX_ZT(64, 1, 16) GFIX_ZT(64, 1, 32)
+  if constexpr (sizeof(R) == 8) {
+    GFIX_ZT(48, 96, 2) GFIX_ZT(48, 96, 1) GFIX_ZT(48, 1, 8) GFIX_ZT(48, 1, 16)
+    GFIX_ZT(32, 1, 8) GFIX_ZT(32, 1, 16) GFIX_ZT(32, 1, 32)
+  }
 #undef GFIX_ZT
   return nullptr;
 }
@@ -179,7 +178,7 @@ class Engine {
   bool odd = false;
   bool coul = false;
   int Lcu = 0;
-  XyFn<F> xy_ct = nullptr;
+  XyFn<F> xy_ct[2] = {nullptr, nullptr};  // forward and inverse
   ZtFn<F> zt_ct = nullptr;
   cudaGraphExec_t gx_cg = nullptr, gx_sd = nullptr;
   cudaGraph_t gr_cg = nullptr, gr_sd = nullptr;  // the same, uninstantiated
@@ -285,38 +284,36 @@ class Engine {
     c.cs_ld = ld;
     // tiles
     c.xy_pitch = c.L[0] + 1;
-    // x columns per zt tile: Landau's (z, t) tiles take 4 where a
-    // compile-time pass for them exists (the autotuner's pick on 16^3x32
-    // and 32^3x64), else 2 (32-byte rows in FP64); Coulomb tiles hold one
-    // slice's z pencils only and take 16
+    // x columns per zt tile: what the register-pencil pass of these extents
+    // takes; else Landau's (z, t) tiles 2 (32-byte rows in FP64) and Coulomb
+    // tiles, which hold one slice's z pencils only, 16
     odd = false;
     for (int a = 0; a < 4; a++)
       for (int k = 0; k < c.ax[a].nstages; k++)
         odd |= (c.ax[a].st[k].r == 5 || c.ax[a].st[k].r == 7);
     const int nt = coul ? 1 : c.L[3];
-    int want_b = coul ? 16 : 2;
-    if (!coul && !odd && c.L[0] % 4 == 0 && ct_zt<F>(c.L[2], nt, 4) != nullptr &&
-        zt_smem(4) <= 200u * 1024u)
-      want_b = 4;
     c.zt_b = 1;
-    for (int b = want_b; b >= 1; b--)
-      if (c.L[0] % b == 0) {
-        c.zt_b = b;
-        break;
+    bool ct_tile = reg_pass(0).fn != nullptr;
+    if (ct_tile) {
+      c.zt_b = reg_pass(0).columns;
+    } else {
+      for (int b = coul ? 16 : 2; b >= 1; b--)
+        if (c.L[0] % b == 0) {
+          c.zt_b = b;
+          break;
+        }
+      // a compile-time pass takes the tile as chosen while its shared memory
+      // fits (tiles up to 16384 elements); the generic passes hold one
+      // element per thread and stage for 8 (16) elements: tiles up to 8192
+      ct_tile = !odd && ct_zt<F>(c.L[2], nt, c.zt_b) != nullptr &&
+                zt_smem(c.zt_b) <= 200u * 1024u;
+      if (!ct_tile) {
+        while (c.zt_b > 1 && (size_t)c.zt_b * c.L[2] * nt > 4096u) c.zt_b /= 2;
+        while (c.zt_b > 1 && c.L[0] % c.zt_b) c.zt_b /= 2;
       }
-    // a compile-time pass takes the tile as chosen while its shared memory
-    // fits (tiles up to 16384 elements); the generic passes hold one
-    // element per thread and stage for 8 (16) elements: tiles up to 8192
-    const bool ct_tile = !odd && ct_zt<F>(c.L[2], nt, c.zt_b) != nullptr &&
-                         zt_smem(c.zt_b) <= 200u * 1024u;
-    if (!ct_tile) {
-      while (c.zt_b > 1 && (size_t)c.zt_b * c.L[2] * nt > 4096u) c.zt_b /= 2;
-      while (c.zt_b > 1 && c.L[0] % c.zt_b) c.zt_b /= 2;
     }
     if ((size_t)c.L[0] * c.L[1] > 8192)
       return fail("FFT xy tile of %d elements exceeds 8192", c.L[0] * c.L[1]);
-    // tile (padded) plus the twiddle tables of its two axes
-    sm_xy = ((size_t)c.xy_pitch * c.L[1] + c.L[0] + c.L[1]) * sizeof(cx<F>);
     // the dynamic shared-memory limit is an attribute of the function, not
     // of a launch: raise it once to the largest tile any engine can use
     if (set_smem_limits()) return -1;
@@ -327,10 +324,8 @@ class Engine {
     if (apply_zt(c.zt_b, ct_tile, 0) && apply_zt(c.zt_b, false, 0))
       return fail("FFT tile of %zu elements exceeds 8192",
                   (size_t)c.zt_b * c.L[2] * nt);
-    g_xy = dim3(V / (c.L[0] * c.L[1]), 4);
     nb_site = (V + kSiteThreads - 1) / kSiteThreads;
-    const size_t nparts =
-        std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y);
+    const size_t nparts = max_parts();
     const size_t groups = tick_groups((unsigned)nparts);
     CK(cudaMalloc(&d_part, (nparts + groups) * 2 * sizeof(double)));
     c.part = d_part;
@@ -368,26 +363,58 @@ class Engine {
     size_t t = (n + pt - 1) / pt;
     return std::max<size_t>(128, (t + 31) / 32 * 32);
   }
-  // the xy pass: compile-time (use_ct) or generic with radix order `order`;
-  // -1 where that pass does not exist for these extents
+  // partials of the widest grid that sums over the lattice: the site kernels',
+  // or an xy pass of one plane of one field per block
+  size_t max_parts() const {
+    return std::max<size_t>((size_t)nb_site, (size_t)c.L[2] * c.L[3] * 4);
+  }
+  // the register-pencil z(,t) pass with tiles of b columns (0: its default)
+  RegZt<F> reg_pass(int b) const {
+    if (!coul) return reg_zt<F>(c.L[2], c.L[3], c.L[0], b);
+    return b > 1 ? RegZt<F>{} : reg_z<F>(c.L[2]);  // (no tiles)
+  }
+  template <typename K>
+  static int shared_limit(K fn, size_t smem) {
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                            (int)cudaSharedmemCarveoutMaxShared));
+    return 0;
+  }
+  // the xy pass: compile-time (use_ct; register pencils, or the staged form
+  // where those do not reach) or generic with radix order `order`; -1 where
+  // that pass does not exist for these extents
   int apply_xy(bool use_ct, int order) {
     for (int a = 0; a < 2; a++)
       if (factorize(c.L[a], c.ax[a], order)) return -1;
     const size_t n = (size_t)c.L[0] * c.L[1];
+    int planes = 1;
+    // tile (padded) plus the twiddle tables of its two axes
+    sm_xy = ((size_t)c.xy_pitch * c.L[1] + c.L[0] + c.L[1]) * sizeof(cx<F>);
     if (use_ct) {
+      const RegXy<F> r = c.L[0] == c.L[1] ? reg_xy<F>(c.L[0], coul ? c.L[2] : c.L[2] * c.L[3])
+                                          : RegXy<F>{};
       XyFn<F> fn = odd ? nullptr : ct_xy<F>(c.L[0], c.L[1]);
-      if (!fn) return -1;
-      xy_ct = fn;
-      bd_xy = ct_threads((int)n);
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sm_xy));
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                              (int)cudaSharedmemCarveoutMaxShared));
+      if (r.fn[0]) {
+        for (int k = 0; k < 2; k++) {
+          xy_ct[k] = r.fn[k];
+          if (shared_limit(r.fn[k], r.smem)) return -1;
+        }
+        bd_xy = r.threads;
+        sm_xy = r.smem;
+        planes = r.planes;
+      } else if (fn) {
+        xy_ct[0] = xy_ct[1] = fn;
+        bd_xy = ct_threads((int)n);
+        if (shared_limit(fn, sm_xy)) return -1;
+      } else {
+        return -1;
+      }
     } else {
-      xy_ct = nullptr;
+      xy_ct[0] = xy_ct[1] = nullptr;
       pt_xy = (n <= 4096u && !odd) ? 8 : 16;
       bd_xy = (int)threads_for(n, pt_xy);
     }
+    g_xy = dim3(V / (int)n / planes, 4);
     xy_plan = use_ct ? -1 : order;
     return 0;
   }
@@ -398,24 +425,32 @@ class Engine {
     for (int a = 2; a < 4; a++)
       if (factorize(c.L[a], c.ax[a], order)) return -1;
     const size_t n = (size_t)b * c.L[2] * nt;
+    g_zt = dim3((c.L[0] / b) * c.L[1] * (coul ? c.L[3] : 1), 4);
     if (use_ct) {
+      const RegZt<F> r = reg_pass(b);
       ZtFn<F> fn = odd ? nullptr : ct_zt<F>(c.L[2], nt, b);
-      if (!fn || zt_smem(b) > 200u * 1024u) return -1;
-      zt_ct = fn;
-      bd_zt = zt_threads<F>((int)n);
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)zt_smem(b)));
-      CK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                              (int)cudaSharedmemCarveoutMaxShared));
+      if (r.fn) {
+        zt_ct = r.fn;
+        bd_zt = r.threads;
+        sm_zt = r.smem;
+        if (coul) g_zt.x = (c.L[0] * c.L[1] + r.threads - 1) / r.threads * c.L[3];
+        if (shared_limit(r.fn, sm_zt)) return -1;
+      } else if (fn && zt_smem(b) <= 200u * 1024u) {
+        zt_ct = fn;
+        bd_zt = ct_threads((int)n);
+        sm_zt = zt_smem(b);
+        if (shared_limit(fn, sm_zt)) return -1;
+      } else {
+        return -1;
+      }
     } else {
       if (n > 8192) return -1;
       zt_ct = nullptr;
       pt_zt = (n <= 4096u && !odd) ? 8 : 16;
       bd_zt = (int)threads_for(n, pt_zt);
+      sm_zt = zt_smem(b);
     }
     c.zt_b = b;
-    sm_zt = zt_smem(b);
-    g_zt = dim3((c.L[0] / b) * c.L[1] * (coul ? c.L[3] : 1), 4);
     zt_plan = use_ct ? -1 : order;
     return 0;
   }
@@ -460,7 +495,7 @@ class Engine {
       if (reset(p)) return -1;
       CK(cudaMemsetAsync(d_F, 0, (size_t)V * 16 * sizeof(cx<F>), s));
       float best = 1e30f, t = 0.f;
-      P = TunedPlan{xy_ct != nullptr, xy_plan < 0 ? 0 : xy_plan, c.zt_b,
+      P = TunedPlan{xy_ct[0] != nullptr, xy_plan < 0 ? 0 : xy_plan, c.zt_b,
                     zt_ct != nullptr, zt_plan < 0 ? 0 : zt_plan, 0.f, 0.f};
       for (int ct = 1; ct >= 0; ct--)
         for (int o = 0; o < (ct ? 1 : kRadixOrders); o++) {
@@ -577,7 +612,7 @@ class Engine {
   }
   void fft_xy(int bwd, int prsum) {
     const Ctx<F> v = cf();
-    const XyFn<F> fn = xy_ct ? xy_ct
+    const XyFn<F> fn = xy_ct[0] ? xy_ct[bwd != 0]
                        : odd ? k_fft_xy<F, 16, true>
                        : pt_xy == 8 ? k_fft_xy<F, 8, false> : k_fft_xy<F, 16, false>;
     launch(fn, g_xy, bd_xy, sm_xy, s, v, bwd, prsum);
@@ -976,7 +1011,7 @@ class Engine {
     CK(cudaMallocHost(&h_sl, sizeof(Slice) * T));
     // per-slice partials: [T][nbs] pairs, next to the engine's own uses
     const size_t need = (size_t)T * nbs;
-    const size_t have = std::max<size_t>((size_t)nb_site, (size_t)g_xy.x * g_xy.y);
+    const size_t have = max_parts();
     if (need > have) {
       cudaFree(d_part);
       d_part = nullptr;
