@@ -193,17 +193,6 @@ __host__ __device__ constexpr int reg_blocks(int threads, int data, size_t smem)
   return n < 1 ? 1 : n > 16 ? 16 : n;
 }
 
-__device__ __forceinline__ void cp_async(void *dst, const void *src, bool wide) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if (wide)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
-}
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
-
 // --- xy planes of N x N ---------------------------------------------------
 // PL planes of one field per block, N threads to each: rows, then columns
 // (k_fft_xy is the generic form).  Resident blocks: as many as hold 128
@@ -224,7 +213,7 @@ __global__ void __launch_bounds__(N *PL, reg_blocks(N *PL, N * sizeof(R) / 2, xy
   const size_t base = (size_t)field * c.V + (size_t)blockIdx.x * (PL * N * N);
   cx<R> *data = pick(c.fb, par) + base;
   for (int e = threadIdx.x; e < PL * N * N; e += PL * N)
-    cp_async(A + (e / N) * P + e % N, data + e, sizeof(R) == 8);
+    cp_async(A + (e / N) * P + e % N, data + e);
   cp_async_wait();
   __syncthreads();
   const int pl = threadIdx.x / N, i = threadIdx.x % N;

@@ -66,6 +66,20 @@ __device__ __forceinline__ cx<R> cscale(cx<R> a, R s) {
   return mk<R>(a.x * s, a.y * s);
 }
 
+// an element fetched to shared memory while the thread goes on (16 or 8
+// bytes), and the wait for all that this thread has under way
+template <typename R>
+__device__ __forceinline__ void cp_async(cx<R> *dst, const cx<R> *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (sizeof(R) == 8)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
 // column Gram-Schmidt of columns 0 (u0,u3,u6) and 1 (u1,u4,u7); column 2
 // from their conjugate cross product.  The normalisations use rsqrt (within
 // an ulp of GLU's 1/sqrt, far cheaper than a division and a square root).
