@@ -15,11 +15,11 @@
 // the psq scale.
 //
 // Per launch at 32^3 x 64: xy 0.070 -> 0.049 ms in FP64 (0.84 of the copy
-// bandwidth), 0.039 -> 0.026 ms in FP32; inverse with sums 0.105 -> 0.091 and
-// 0.069 -> 0.066 ms; (z, t) 0.167 -> 0.162 and 0.094 -> 0.066 ms.  FP32 at 48^3
-// x 96: 0.260 -> 0.133, 0.437 -> 0.317 and 0.780 -> 0.622 ms.  FP64 at 20^3 x
+// bandwidth), 0.039 -> 0.026 ms in FP32; inverse with sums 0.105 -> 0.087 and
+// 0.069 -> 0.053 ms; (z, t) 0.167 -> 0.162 and 0.094 -> 0.066 ms.  FP32 at 48^3
+// x 96: 0.260 -> 0.133, 0.437 -> 0.246 and 0.780 -> 0.622 ms.  FP64 at 20^3 x
 // 40, where only the generic passes served: 0.070 + 0.120 + 0.082 -> 0.014 +
-// 0.022 + 0.029 ms.  The register budget ends it: pencils of 64 in FP32 and 32
+// 0.022 + 0.024 ms.  The register budget ends it: pencils of 64 in FP32 and 32
 // in FP64, Coulomb z pencils (no shared memory to share the work) of 48 and
 // 24 (0.072 against 0.069 ms with 32 in FP64); beyond, fft_ct.cuh.
 //
@@ -227,41 +227,40 @@ __global__ void __launch_bounds__(N *PL, reg_blocks(N *PL, N * sizeof(R) / 2, xy
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < N; k++) v[k] = tile[k * P + i];
+  constexpr bool RAG = N * PL % 32 != 0;
+  // the previous field, for the sums, on its way into the tile meanwhile
+  // (32^3 x 64: 0.087 ms, FP32 0.053; loaded by the sums themselves 0.090 and
+  // 0.066, 16^3 x 32 0.015 and 0.013 against 0.019 and 0.016)
+  const bool sums = B && prsum;
+  if (sums) {
+    const cx<R> *old = pick(c.fb, par ^ 1) + base;
+    __syncthreads();
+    for (int e = threadIdx.x; e < PL * N * N; e += PL * N)
+      cp_async(A + (e / N) * P + e % N, old + e);
+  }
   reg_fft<R, N, B>(v);
   data += (size_t)pl * N * N + i;
-  // with sums: FP64 takes them and the ticket, whose fence would wait for the
-  // stores, before the stores; FP32 after them, in a loop that keeps few loads
-  // in flight and its registers for more blocks (32^3 x 64: FP32 0.066 ms,
-  // 0.071 unrolled; FP64 0.091 ms, 0.098 after the stores)
-  constexpr bool RAG = N * PL % 32 != 0, LATE = !B || sizeof(R) == 4;
-  if constexpr (LATE) {
 #pragma unroll
-    for (int k = 0; k < N; k++) data[k * N] = v[k];
-  }
-  if constexpr (B) {
+  for (int k = 0; k < N; k++) data[k * N] = v[k];
+  if (sums) {
     double s[2] = {0.0, 0.0};
-    if (prsum) {
-      const cx<R> *old = pick(c.fb, par ^ 1) + base + (size_t)pl * N * N + i;
-#pragma unroll(LATE ? 8 : N)
-      for (int k = 0; k < N; k++) {
-        const cx<R> od = old[k * N];
-        const double a = v[k].x, b = v[k].y;
-        const double tr = a - (double)od.x, ti = b - (double)od.y;
-        if (field == 0) {
-          s[0] += 2.0 * (a * a + b * b + a * b);
-          s[1] += 2.0 * (a * tr + b * ti) + (a * ti + b * tr);
-        } else {
-          s[0] += 2.0 * (a * a + b * b);
-          s[1] += 2.0 * (a * tr + b * ti);
-        }
-      }
-      xy_sums_begin<RAG>(c, s);
-    }
-    if constexpr (!LATE) {
+    cp_async_wait();
+    __syncthreads();
 #pragma unroll
-      for (int k = 0; k < N; k++) data[k * N] = v[k];
+    for (int k = 0; k < N; k++) {
+      const cx<R> od = tile[k * P + i];
+      const double a = v[k].x, b = v[k].y;
+      const double tr = a - (double)od.x, ti = b - (double)od.y;
+      if (field == 0) {
+        s[0] += 2.0 * (a * a + b * b + a * b);
+        s[1] += 2.0 * (a * tr + b * ti) + (a * ti + b * tr);
+      } else {
+        s[0] += 2.0 * (a * a + b * b);
+        s[1] += 2.0 * (a * tr + b * ti);
+      }
     }
-    if (prsum) xy_sums<RAG>(c, s);
+    xy_sums_begin<RAG>(c, s);
+    xy_sums<RAG>(c, s);
   }
 }
 
