@@ -12,12 +12,12 @@
 // Coulomb slices, whose pencils neighbouring threads read in full lines.
 // A t axis too long for one thread is split over two, t = 2n + h, which
 // exchange half of their elements by shuffles (radix 2) on either side of
-// the psq scale.
+// the psq scale; the longest z and t axes over two and four.
 //
 // Per launch at 32^3 x 64: xy 0.070 -> 0.049 ms in FP64 (0.84 of the copy
 // bandwidth), 0.039 -> 0.026 ms in FP32; inverse with sums 0.105 -> 0.087 and
-// 0.069 -> 0.053 ms; (z, t) 0.167 -> 0.162 and 0.094 -> 0.066 ms.  FP32 at 48^3
-// x 96: 0.260 -> 0.133, 0.437 -> 0.246 and 0.780 -> 0.622 ms.  FP64 at 20^3 x
+// 0.069 -> 0.053 ms; (z, t) 0.167 -> 0.157 and 0.094 -> 0.066 ms.  FP32 at 48^3
+// x 96: 0.260 -> 0.133, 0.437 -> 0.246 and 0.780 -> 0.492 ms.  FP64 at 20^3 x
 // 40, where only the generic passes served: 0.070 + 0.120 + 0.082 -> 0.014 +
 // 0.022 + 0.024 ms.  The register budget ends it: pencils of 64 in FP32 and 32
 // in FP64, Coulomb z pencils (no shared memory to share the work) of 48 and
@@ -193,6 +193,43 @@ __host__ __device__ constexpr int reg_blocks(int threads, int data, size_t smem)
   return n < 1 ? 1 : n > 16 ? 16 : n;
 }
 
+// --- pencils shared by lanes ------------------------------------------------
+// Radix-2 steps between lanes D apart of which h = 0 holds the even and h = 1
+// the odd half of an N-point transform, v[i] at some k of N/2 each.  Forward:
+// X[k] = E[k] + W^k O[k] and X[k + N/2] = E[k] - W^k O[k] for half of the k, to
+// v[j] and v[j + Q]; k = j + h N/4, or j + h8 N/8 + h N/4 after a step before.
+template <typename R, int N, int Q, int D>
+__device__ __forceinline__ void lane_fwd(cx<R> (&v)[2 * Q], int h, int h8 = 0) {
+  static_for<Q>([&](auto J) {
+    constexpr int j = J;
+    const cx<R> snd = h ? v[j] : v[j + Q];
+    const cx<R> rcv = mk<R>(__shfl_xor_sync(0xffffffffu, snd.x, D),
+                            __shfl_xor_sync(0xffffffffu, snd.y, D));
+    const cx<R> e = h ? rcv : v[j];
+    cx<R> o = rot<R, j, N, false>(h ? v[j + Q] : rcv);
+    if (h8) o = rot<R, 1, 8, false>(o);
+    if (h) o = mk<R>(o.y, -o.x);
+    v[j] = cadd(e, o);
+    v[j + Q] = csub(e, o);
+  });
+}
+// back: E' = X[k] + X[k + N/2], O' = (X[k] - X[k + N/2]) W^-k
+template <typename R, int N, int Q, int D>
+__device__ __forceinline__ void lane_bwd(cx<R> (&v)[2 * Q], int h, int h8 = 0) {
+  static_for<Q>([&](auto J) {
+    constexpr int j = J;
+    const cx<R> s = cadd(v[j], v[j + Q]);
+    cx<R> d = rot<R, j, N, true>(csub(v[j], v[j + Q]));
+    if (h8) d = rot<R, 1, 8, true>(d);
+    if (h) d = mk<R>(-d.y, d.x);
+    const cx<R> out = h ? s : d;
+    const cx<R> in = mk<R>(__shfl_xor_sync(0xffffffffu, out.x, D),
+                           __shfl_xor_sync(0xffffffffu, out.y, D));
+    v[j] = h ? in : s;
+    v[j + Q] = h ? d : in;
+  });
+}
+
 // --- xy planes of N x N ---------------------------------------------------
 // PL planes of one field per block, N threads to each: rows, then columns
 // (k_fft_xy is the generic form).  Resident blocks: as many as hold 128
@@ -271,7 +308,7 @@ __device__ __forceinline__ R psq_of(double kcos, double D, double maxp) {
   return (R)(maxp * __drcp_rn(p2));
 }
 
-// --- z and t of a tile of BW x columns, W of them at a time ----------------
+// --- z and t of a tile of BW x columns --------------------------------------
 template <typename R, int LT>
 constexpr bool zt_split = LT > kRegMax<R>;
 template <typename R, int LZ, int LT, int BW>
@@ -291,109 +328,178 @@ __host__ __device__ constexpr int zt_reg_blocks() {
                     zt_reg_smem<R, LZ, LT, BW>());
 }
 
-template <typename R, int LZ, int LT, int BW, int W = BW>
-__global__ void __launch_bounds__(zt_reg_threads<R, LZ, LT, W>(),
-                                  zt_reg_blocks<R, LZ, LT, W>())
+template <typename R, int LZ, int LT, int BW>
+__global__ void __launch_bounds__(zt_reg_threads<R, LZ, LT, BW>(),
+                                  zt_reg_blocks<R, LZ, LT, BW>())
     k_fft_zt_reg(Ctx<R> c) {
   if (c.st->done) return;
-  constexpr int TS = LZ * W + zt_pad(W), NT = zt_reg_threads<R, LZ, LT, W>();
-  constexpr int NPZ = LT * W, NPT = LZ * W;
+  constexpr int TS = LZ * BW + zt_pad(BW), NT = zt_reg_threads<R, LZ, LT, BW>();
+  constexpr int NPZ = LT * BW, NPT = LZ * BW;
+  extern __shared__ unsigned char smem_raw[];
+  cx<R> *A = reinterpret_cast<cx<R> *>(smem_raw);
+  const int nxb = c.L[0] / BW;
+  const int y = blockIdx.x / nxb;
+  const size_t sz = (size_t)c.L[0] * c.L[1];
+  const int x0 = blockIdx.x % nxb * BW;
+  cx<R> *data = pick(c.fb, c.st->parity) + (size_t)blockIdx.y * c.V + (size_t)c.L[0] * y + x0;
+  const double cxy = c.cs[c.cs_ld + y];
+  const double *cz = c.cs + 2 * c.cs_ld, *ct = c.cs + 3 * c.cs_ld;
+#pragma unroll 1
+  for (int p = threadIdx.x; p < NPZ; p += NT) {
+    const int b = p % BW, t = p / BW;
+    const cx<R> *g = data + b + sz * (LZ * t);
+    cx<R> v[LZ];
+#pragma unroll
+    for (int k = 0; k < LZ; k++) v[k] = g[sz * k];
+    reg_fft<R, LZ, false>(v);
+#pragma unroll
+    for (int k = 0; k < LZ; k++) A[b + BW * k + TS * t] = v[k];
+  }
+  __syncthreads();
+  if constexpr (!zt_split<R, LT>) {
+    const int p = threadIdx.x;
+    if (p < NPT) {
+      const double k3 = c.cs[x0 + p % BW] + cxy + cz[p / BW];
+      cx<R> v[LT];
+#pragma unroll
+      for (int t = 0; t < LT; t++) v[t] = A[p + TS * t];
+      reg_fft<R, LT, false>(v);
+#pragma unroll
+      for (int t = 0; t <= LT / 2; t++) {  // psq is even in t
+        const R f = psq_of<R>(k3 + ct[t], 4.0, c.maxp);
+        v[t] = cscale(v[t], f);
+        if (t > 0 && 2 * t < LT) v[LT - t] = cscale(v[LT - t], f);
+      }
+      reg_fft<R, LT, true>(v);
+#pragma unroll
+      for (int t = 0; t < LT; t++) A[p + TS * t] = v[t];
+    }
+  } else {
+    // lanes 0-15 the even, 16-31 the odd t of 16 pencils
+    constexpr int H = LT / 2, Q = H / 2;
+    static_assert(LT % 4 == 0 && H <= kRegMax<R>, "split t axis");
+    const int h = (threadIdx.x >> 4) & 1;
+    const int p = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15);
+    const bool on = p < NPT;
+    const int pc = on ? p : 0;
+    const double k3 = c.cs[x0 + pc % BW] + cxy + cz[pc / BW];
+    cx<R> v[H];
+#pragma unroll
+    for (int n = 0; n < H; n++) v[n] = A[pc + TS * (2 * n + h)];
+    reg_fft<R, H, false>(v);
+    // X[k] = E[k] + W^k O[k], X[k + H] = E[k] - W^k O[k] for k = j + h Q
+    static_for<Q>([&](auto J) {
+      constexpr int j = J;
+      const cx<R> snd = h ? v[j] : v[j + Q];
+      const cx<R> rcv = mk<R>(__shfl_xor_sync(0xffffffffu, snd.x, 16),
+                              __shfl_xor_sync(0xffffffffu, snd.y, 16));
+      const cx<R> e = h ? rcv : v[j];
+      cx<R> o = rot<R, j, LT, false>(h ? v[j + Q] : rcv);
+      if (h) o = mk<R>(o.y, -o.x);  // W^Q = -i
+      const R f0 = psq_of<R>(k3 + ct[j + h * Q], 4.0, c.maxp);
+      const R f1 = psq_of<R>(k3 + ct[j + h * Q + H], 4.0, c.maxp);
+      const cx<R> a = cscale(cadd(e, o), f0), b = cscale(csub(e, o), f1);
+      // back: E' = X[k] + X[k + H], O' = (X[k] - X[k + H]) W^-k
+      const cx<R> s = cadd(a, b);
+      cx<R> d = rot<R, j, LT, true>(csub(a, b));
+      if (h) d = mk<R>(-d.y, d.x);
+      const cx<R> out = h ? s : d;
+      const cx<R> in = mk<R>(__shfl_xor_sync(0xffffffffu, out.x, 16),
+                             __shfl_xor_sync(0xffffffffu, out.y, 16));
+      v[j] = h ? in : s;
+      v[j + Q] = h ? d : in;
+    });
+    reg_fft<R, H, true>(v);
+    if (on) {
+#pragma unroll
+      for (int n = 0; n < H; n++) A[p + TS * (2 * n + h)] = v[n];
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int p = threadIdx.x; p < NPZ; p += NT) {
+    const int b = p % BW, t = p / BW;
+    cx<R> v[LZ];
+#pragma unroll
+    for (int k = 0; k < LZ; k++) v[k] = A[b + BW * k + TS * t];
+    reg_fft<R, LZ, true>(v);
+    cx<R> *g = data + b + sz * (LZ * t);
+#pragma unroll
+    for (int k = 0; k < LZ; k++) g[sz * k] = v[k];
+  }
+}
+
+// --- z over two and t over four threads, W of the BW columns at a time ------
+// For axes whose pencils leave a thread too few registers or a block too few
+// warps: a thread holds a quarter of a t pencil, so that tiles of 32-byte rows
+// and twice the warps fit.  Per launch at n^3 x 2n, before (fft_ct, generic
+// for 36 and 40; FP32 two threads a t pencil, 2 columns) and now: FP64 48: 1.38
+// -> 0.955 ms, 40: 2.00 -> 0.458, 36: 1.13 -> 0.345, 32: 0.162 -> 0.157; FP32
+// 48: 0.627 -> 0.492, 40: 0.307 -> 0.229, 36: 0.193 -> 0.155.  Shorter axes lose
+// more to the shuffles: FP32 32 0.078 against 0.066 ms, FP64 24 0.044 against
+// 0.034, 28 equal.
+template <typename R, int LZ, int LT, int W>
+__host__ __device__ constexpr int zt_quad_blocks() {
+  return reg_blocks(4 * LZ * W, LZ / 2 * sizeof(R) / 2, zt_reg_smem<R, LZ, LT, W>());
+}
+template <typename R, int LZ, int LT, int BW, int W = BW>
+__global__ void __launch_bounds__(4 * LZ * W, zt_quad_blocks<R, LZ, LT, W>())
+    k_fft_zt_quad(Ctx<R> c) {
+  static_assert(LT == 2 * LZ && LZ % 4 == 0 && LZ * W % 8 == 0, "whole warps");
+  if (c.st->done) return;
+  constexpr int TS = LZ * W + zt_pad(W), M = LZ / 2, Q = M / 2;
   extern __shared__ unsigned char smem_raw[];
   cx<R> *A = reinterpret_cast<cx<R> *>(smem_raw);
   const int nxb = c.L[0] / BW;
   const int y = blockIdx.x / nxb;
   const size_t sz = (size_t)c.L[0] * c.L[1];
   cx<R> *row = pick(c.fb, c.st->parity) + (size_t)blockIdx.y * c.V + (size_t)c.L[0] * y;
-  const double cxy = c.cs[c.cs_ld + y];
-  const double *cz = c.cs + 2 * c.cs_ld, *ct = c.cs + 3 * c.cs_ld;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // z: lanes 0-15 the even, 16-31 the odd z of 16 pencils (b, t)
+  const int zh = lane >> 4, zp = w * 16 + (lane & 15), zb = zp % W, zt = zp / W;
+  cx<R> *const Az = A + zb + TS * zt;
+  // t: t = 4 n + 2 h0 + h1 of 8 pencils (b, z)
+  const int h0 = (lane >> 3) & 1, h1 = lane >> 4, tp = w * 8 + (lane & 7);
+  cx<R> *const At = A + tp + TS * (2 * h0 + h1);
 #pragma unroll 1
   for (int sub = 0; sub < BW / W; sub++) {
     const int x0 = blockIdx.x % nxb * BW + sub * W;
-    cx<R> *data = row + x0;
+    cx<R> *const g = row + x0 + zb + sz * (LZ * zt + zh);
     if (sub) __syncthreads();
-#pragma unroll 1
-    for (int p = threadIdx.x; p < NPZ; p += NT) {
-      const int b = p % W, t = p / W;
-      const cx<R> *g = data + b + sz * (LZ * t);
-      cx<R> v[LZ];
+    cx<R> v[M];
 #pragma unroll
-      for (int k = 0; k < LZ; k++) v[k] = g[sz * k];
-      reg_fft<R, LZ, false>(v);
+    for (int n = 0; n < M; n++) v[n] = g[sz * (2 * n)];
+    reg_fft<R, M, false>(v);
+    lane_fwd<R, LZ, Q, 16>(v, zh);
 #pragma unroll
-      for (int k = 0; k < LZ; k++) A[b + W * k + TS * t] = v[k];
-    }
+    for (int i = 0; i < M; i++) Az[W * (i % Q + i / Q * M + zh * Q)] = v[i];
     __syncthreads();
-    if constexpr (!zt_split<R, LT>) {
-      const int p = threadIdx.x;
-      if (p < NPT) {
-        const double k3 = c.cs[x0 + p % W] + cxy + cz[p / W];
-        cx<R> v[LT];
 #pragma unroll
-        for (int t = 0; t < LT; t++) v[t] = A[p + TS * t];
-        reg_fft<R, LT, false>(v);
+    for (int n = 0; n < M; n++) v[n] = At[TS * 4 * n];
+    reg_fft<R, M, false>(v);
+    lane_fwd<R, 2 * M, Q, 8>(v, h0);
+    lane_fwd<R, 4 * M, Q, 16>(v, h1, h0);
+    {
+      const double k3 = c.cs[x0 + tp % W] + c.cs[c.cs_ld + y] + c.cs[2 * c.cs_ld + tp / W];
+      const double *ct = c.cs + 3 * c.cs_ld + Q * h0 + 2 * Q * h1;
 #pragma unroll
-        for (int t = 0; t <= LT / 2; t++) {  // psq is even in t
-          const R f = psq_of<R>(k3 + ct[t], 4.0, c.maxp);
-          v[t] = cscale(v[t], f);
-          if (t > 0 && 2 * t < LT) v[LT - t] = cscale(v[LT - t], f);
-        }
-        reg_fft<R, LT, true>(v);
-#pragma unroll
-        for (int t = 0; t < LT; t++) A[p + TS * t] = v[t];
-      }
-    } else {
-      // lanes 0-15 the even, 16-31 the odd t of 16 pencils
-      constexpr int H = LT / 2, Q = H / 2;
-      static_assert(LT % 4 == 0 && H <= kRegMax<R>, "split t axis");
-      const int h = (threadIdx.x >> 4) & 1;
-      const int p = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15);
-      const bool on = p < NPT;
-      const int pc = on ? p : 0;
-      const double k3 = c.cs[x0 + pc % W] + cxy + cz[pc / W];
-      cx<R> v[H];
-#pragma unroll
-      for (int n = 0; n < H; n++) v[n] = A[pc + TS * (2 * n + h)];
-      reg_fft<R, H, false>(v);
-      // X[k] = E[k] + W^k O[k], X[k + H] = E[k] - W^k O[k] for k = j + h Q
-      static_for<Q>([&](auto J) {
-        constexpr int j = J;
-        const cx<R> snd = h ? v[j] : v[j + Q];
-        const cx<R> rcv = mk<R>(__shfl_xor_sync(0xffffffffu, snd.x, 16),
-                                __shfl_xor_sync(0xffffffffu, snd.y, 16));
-        const cx<R> e = h ? rcv : v[j];
-        cx<R> o = rot<R, j, LT, false>(h ? v[j + Q] : rcv);
-        if (h) o = mk<R>(o.y, -o.x);  // W^Q = -i
-        const R f0 = psq_of<R>(k3 + ct[j + h * Q], 4.0, c.maxp);
-        const R f1 = psq_of<R>(k3 + ct[j + h * Q + H], 4.0, c.maxp);
-        const cx<R> a = cscale(cadd(e, o), f0), b = cscale(csub(e, o), f1);
-        // back: E' = X[k] + X[k + H], O' = (X[k] - X[k + H]) W^-k
-        const cx<R> s = cadd(a, b);
-        cx<R> d = rot<R, j, LT, true>(csub(a, b));
-        if (h) d = mk<R>(-d.y, d.x);
-        const cx<R> out = h ? s : d;
-        const cx<R> in = mk<R>(__shfl_xor_sync(0xffffffffu, out.x, 16),
-                               __shfl_xor_sync(0xffffffffu, out.y, 16));
-        v[j] = h ? in : s;
-        v[j + Q] = h ? d : in;
-      });
-      reg_fft<R, H, true>(v);
-      if (on) {
-#pragma unroll
-        for (int n = 0; n < H; n++) A[p + TS * (2 * n + h)] = v[n];
+      for (int i = 0; i < M; i++) {
+        v[i] = cscale(v[i], psq_of<R>(k3 + ct[i % Q + i / Q * (2 * M)], 4.0, c.maxp));
+        if (i % 4 == 3) asm volatile("" ::: "memory");  // (not all cosines at once)
       }
     }
+    lane_bwd<R, 4 * M, Q, 16>(v, h1, h0);
+    lane_bwd<R, 2 * M, Q, 8>(v, h0);
+    reg_fft<R, M, true>(v);
+#pragma unroll
+    for (int n = 0; n < M; n++) At[TS * 4 * n] = v[n];
     __syncthreads();
-#pragma unroll 1
-    for (int p = threadIdx.x; p < NPZ; p += NT) {
-      const int b = p % W, t = p / W;
-      cx<R> v[LZ];
 #pragma unroll
-      for (int k = 0; k < LZ; k++) v[k] = A[b + W * k + TS * t];
-      reg_fft<R, LZ, true>(v);
-      cx<R> *g = data + b + sz * (LZ * t);
+    for (int i = 0; i < M; i++) v[i] = Az[W * (i % Q + i / Q * M + zh * Q)];
+    lane_bwd<R, LZ, Q, 16>(v, zh);
+    reg_fft<R, M, true>(v);
 #pragma unroll
-      for (int k = 0; k < LZ; k++) g[sz * k] = v[k];
-    }
+    for (int n = 0; n < M; n++) g[sz * (2 * n)] = v[n];
   }
 }
 

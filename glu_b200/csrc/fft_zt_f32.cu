@@ -7,14 +7,21 @@ namespace gfix {
 template <>
 RegZt<float> reg_zt<float>(int lz, int lt, int lx, int want) {
   RegZt<float> r;
-#define GFIX_T(LZ, LT, B) GFIX_TW(LZ, LT, B, B)
-#define GFIX_TW(LZ, LT, B, W)                                                       \
+#define GFIX_T(LZ, LT, B)                                                           \
   if (lz == LZ && lt == LT && lx % B == 0 && (want ? want == B : !r.fn)) {          \
-    r.fn = k_fft_zt_reg<float, LZ, LT, B, W>;                                       \
+    r.fn = k_fft_zt_reg<float, LZ, LT, B>;                                       \
     r.columns = B;                                                                  \
-    r.threads = zt_reg_threads<float, LZ, LT, W>();                                \
+    r.threads = zt_reg_threads<float, LZ, LT, B>();                                \
+    r.smem = zt_reg_smem<float, LZ, LT, B>();                                      \
+  }
+#define GFIX_Q(LZ, LT, B, W)                                                        \
+  if (lz == LZ && lt == LT && lx % B == 0 && (want ? want == B : !r.fn)) {          \
+    r.fn = k_fft_zt_quad<float, LZ, LT, B, W>;                                     \
+    r.columns = B;                                                                  \
+    r.threads = 4 * LZ * W;                                                         \
     r.smem = zt_reg_smem<float, LZ, LT, W>();                                      \
   }
+  GFIX_Q(36, 72, 4, 4) GFIX_Q(40, 80, 4, 4) GFIX_Q(48, 96, 4, 4)
   GFIX_T(4, 4, 4) GFIX_T(4, 8, 4) GFIX_T(8, 8, 4) GFIX_T(8, 16, 4) GFIX_T(12, 12, 4)
   GFIX_T(12, 24, 4) GFIX_T(16, 16, 4) GFIX_T(16, 32, 4) GFIX_T(20, 20, 4) GFIX_T(20, 40, 4)
   GFIX_T(24, 24, 4) GFIX_T(24, 48, 4) GFIX_T(4, 4, 2) GFIX_T(4, 8, 2) GFIX_T(8, 8, 2)
@@ -25,8 +32,8 @@ RegZt<float> reg_zt<float>(int lz, int lt, int lx, int want) {
   GFIX_T(28, 56, 4) GFIX_T(32, 64, 4) GFIX_T(32, 64, 2) GFIX_T(32, 64, 1)
   GFIX_T(18, 36, 2) GFIX_T(30, 60, 2) GFIX_T(36, 36, 2) GFIX_T(36, 72, 2) GFIX_T(40, 40, 2)
   GFIX_T(40, 80, 2) GFIX_T(48, 48, 2) GFIX_T(48, 96, 2) GFIX_T(48, 96, 1)
+#undef GFIX_Q
 #undef GFIX_T
-#undef GFIX_TW
   return r;
 }
 

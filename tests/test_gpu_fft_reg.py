@@ -1,5 +1,5 @@
 """The register-pencil FFT passes at every kind of extent they are compiled
-for (one- and two-thread t axes, whole and partial blocks, radices 2 to 7),
+for (axes of one to four threads, whole and partial blocks, radices 2 to 7),
 against numpy's transform in 64 bits."""
 import numpy as np
 import pytest
@@ -31,7 +31,8 @@ def _accelerate(f, dims, nd):
     (4, 4, 4, 4), (4, 4, 4, 8), (6, 6, 6, 12), (8, 8, 8, 16), (10, 10, 10, 20), (12, 12, 12, 24),
     (14, 14, 14, 28), (16, 16, 16, 32), (18, 18, 18, 36), (20, 20, 20, 40), (24, 24, 24, 48),
     (28, 28, 28, 28), (28, 28, 28, 56), (30, 30, 30, 60), (32, 32, 32, 32), (32, 32, 32, 64),
-    (6, 6, 32, 64), (5, 5, 32, 64), (10, 10, 5, 3)])
+    (6, 6, 32, 64), (5, 5, 32, 64), (8, 4, 48, 96), (5, 6, 48, 96),
+    (8, 4, 36, 72), (8, 4, 40, 80), (36, 36, 4, 4), (40, 40, 6, 3), (64, 64, 3, 2), (10, 10, 5, 3)])
 def test_landau_transform(dims):
     rng = np.random.default_rng(1)
     V = int(np.prod(dims))
@@ -56,7 +57,8 @@ def test_coulomb_transform(dims):
 
 @pytest.mark.parametrize("dims", [(6, 6, 6, 12), (10, 10, 10, 10), (18, 18, 18, 36),
                                   (20, 20, 20, 40), (36, 36, 36, 36), (40, 40, 40, 80),
-                                  (48, 48, 48, 48), (4, 4, 48, 96), (5, 5, 48, 96), (64, 64, 2, 2)])
+                                  (48, 48, 48, 48), (4, 4, 48, 96), (8, 8, 32, 64), (5, 5, 48, 96),
+                                  (8, 8, 36, 72), (64, 64, 2, 2)])
 def test_fp32_passes_follow_fp64(dims):
     """One steepest-descent step in each phase of a mixed fix (FP32 fields in
     both) against two FP64 ones: links to FP32 rounding of the directions."""
