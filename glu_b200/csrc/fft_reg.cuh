@@ -20,7 +20,8 @@
 // x 96: 0.260 -> 0.133, 0.437 -> 0.246 and 0.780 -> 0.492 ms.  FP64 at 20^3 x
 // 40, where only the generic passes served: 0.070 + 0.120 + 0.082 -> 0.014 +
 // 0.022 + 0.024 ms.  The register budget ends it: pencils of 64 in FP32 and 32
-// in FP64, Coulomb z pencils (no shared memory to share the work) of 48 and
+// in FP64 (planes of up to 64 by two lanes a
+// pencil), Coulomb z pencils (no shared memory to share the work) of 48 and
 // 24 (0.072 against 0.069 ms with 32 in FP64); beyond, fft_ct.cuh.
 //
 // Included by the FFT translation units (fft_xy_f32.cu .. fft_zt_f64.cu) only.
@@ -298,6 +299,85 @@ __global__ void __launch_bounds__(N *PL, reg_blocks(N *PL, N * sizeof(R) / 2, xy
     }
     xy_sums_begin<RAG>(c, s);
     xy_sums<RAG>(c, s);
+  }
+}
+
+// --- xy planes of N x N, each pencil shared by two lanes --------------------
+// For FP64 planes beyond 32: half a pencil fits a thread where a whole one
+// doesn't.  Per launch, forward and inverse with sums, before (fft_ct; 36 and
+// 40 generic) and now: 36^3 x 72 0.454 + 0.525 -> 0.086 + 0.130 ms, 40^3 x 80
+// 0.690 + 0.798 -> 0.115 + 0.174, 48^3 x 96 0.480 + 0.700 -> 0.210 + 0.332 (0.94
+// to 0.99 of the copy bandwidth), Coulomb 64^3 x 16 0.174 + 0.249 -> 0.097 +
+// 0.139.
+template <typename R, int N, int PL, bool B>
+__global__ void __launch_bounds__(2 * N *PL, reg_blocks(2 * N *PL, N *sizeof(R) / 4 - 4,
+                                                        xy_reg_smem<R, N, PL>()))
+    k_fft_xy_pair(Ctx<R> c, int, int prsum) {
+  static_assert(N % 4 == 0 && N * PL % 16 == 0, "whole warps");
+  if (xy_done(c, B)) return;
+  if (c.skip && c.skip[blockIdx.x / (gridDim.x / c.L[3])]) return;  // finished slice
+  extern __shared__ unsigned char smem_raw[];
+  constexpr int P = N + 1, NT = 2 * N * PL, M = N / 2, Q = M / 2;
+  cx<R> *A = reinterpret_cast<cx<R> *>(smem_raw);
+  const int field = blockIdx.y, par = c.st->parity;
+  const size_t base = (size_t)field * c.V + (size_t)blockIdx.x * (PL * N * N);
+  cx<R> *data = pick(c.fb, par) + base;
+  for (int e = threadIdx.x; e < PL * N * N; e += NT) cp_async(A + (e / N) * P + e % N, data + e);
+  cp_async_wait();
+  __syncthreads();
+  // lanes 0-15 the even, 16-31 the odd elements of 16 pencils (plane, i); the
+  // transform's other side at k = j + h Q and k + M
+  const int h = (threadIdx.x >> 4) & 1, q = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15);
+  const int pl = q / N, i = q % N;
+  cx<R> *tile = A + pl * (P * N);
+  auto pos = [&](int n, bool freq) { return freq ? n % Q + n / Q * M + h * Q : 2 * n + h; };
+  cx<R> v[M];
+  auto fft = [&]() {
+    if constexpr (!B) {
+      reg_fft<R, M, false>(v);
+      lane_fwd<R, N, Q, 16>(v, h);
+    } else {
+      lane_bwd<R, N, Q, 16>(v, h);
+      reg_fft<R, M, true>(v);
+    }
+  };
+#pragma unroll
+  for (int n = 0; n < M; n++) v[n] = tile[i * P + pos(n, B)];
+  fft();
+#pragma unroll
+  for (int n = 0; n < M; n++) tile[i * P + pos(n, !B)] = v[n];
+  __syncthreads();
+#pragma unroll
+  for (int n = 0; n < M; n++) v[n] = tile[pos(n, B) * P + i];
+  const bool sums = B && prsum;
+  if (sums) {
+    const cx<R> *old = pick(c.fb, par ^ 1) + base;
+    __syncthreads();
+    for (int e = threadIdx.x; e < PL * N * N; e += NT) cp_async(A + (e / N) * P + e % N, old + e);
+  }
+  fft();
+  data += (size_t)pl * N * N + i;
+#pragma unroll
+  for (int n = 0; n < M; n++) data[pos(n, !B) * N] = v[n];
+  if (sums) {
+    double s[2] = {0.0, 0.0};
+    cp_async_wait();
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < M; n++) {
+      const cx<R> od = tile[pos(n, !B) * P + i];
+      const double a = v[n].x, b = v[n].y;
+      const double tr = a - (double)od.x, ti = b - (double)od.y;
+      if (field == 0) {
+        s[0] += 2.0 * (a * a + b * b + a * b);
+        s[1] += 2.0 * (a * tr + b * ti) + (a * ti + b * tr);
+      } else {
+        s[0] += 2.0 * (a * a + b * b);
+        s[1] += 2.0 * (a * tr + b * ti);
+      }
+    }
+    xy_sums_begin<false>(c, s);
+    xy_sums<false>(c, s);
   }
 }
 

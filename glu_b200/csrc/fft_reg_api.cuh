@@ -1,7 +1,7 @@
 // The register-pencil passes (fft_reg.cuh) by extents.  They are compiled in
 // translation units of their own, one for each pass and type (fft_xy_f32.cu
-// .. fft_zt_f64.cu), for the extents listed there: 4 to 32, in FP32 some up
-// to 64, and t axes of once or twice the z extent.
+// .. fft_zt_f64.cu), for the extents listed there: 4 to 32, some up to
+// 64, and t axes of once or twice the z extent.
 #pragma once
 
 #include "kernels.cuh"
