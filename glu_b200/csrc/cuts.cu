@@ -869,7 +869,6 @@ struct Work {
   int pt_xy = 8, pt_zt = 8, bd_xy = 128, bd_zt = 128;
   size_t sm_xy = 0, sm_zt = 0;
   bool odd = false;
-  int sms = 0;  // of the device
   // compile-time passes, if any: xy_fn[definition] (LINEAR, LOG)
   CutFn xy_fn[2] = {nullptr, nullptr}, zt_fn = nullptr;
   bool xy4 = false;  // xy_fn are k_cut_xy4_ct (the Lie fields computed inside)
@@ -906,9 +905,6 @@ struct Work {
     }
     if (Vs > (size_t)INT32_MAX / 4) return cfail("lattice volume %zu too large", Vs);
     V = (int)Vs;
-    int dev = 0;
-    CCK(cudaGetDevice(&dev));
-    CCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     for (int i = 0; i < 4; i++) {
       if (factorize(L[i], c.ax[i]) != 0)
         return cfail("extent %d has a prime factor above %d", L[i], kMaxRadix);
@@ -1031,13 +1027,10 @@ struct Work {
   // quarter of an xy plane (the fields they leave then fit in d_F, three
   // times): both passes take 0.197 against 0.459 ms with 81 of 400 components
   // (20^3 x 40), 0.858 against 1.274 ms with 81 of 1024 (32^3 x 64), but 0.090
-  // against 0.084 ms with 81 of 256 (16^3 x 32).  A block takes all four
-  // directions of an xy plane, so that they need two planes an SM to fill the
-  // GPU (20 x 6 x 6 x 12 with logarithms: a call 0.64 against 0.52 ms).  Their
-  // rows must be short enough for a chunk of them in shared memory.
+  // against 0.084 ms with 81 of 256 (16^3 x 32).  Their rows must be short
+  // enough for a chunk of them in shared memory.
   bool partial(const MomList &ml) const {
-    return 4 * ml.K[0] * ml.K[1] <= L[0] * L[1] && L[2] * L[3] >= 2 * sms &&
-           L[0] <= 2 * kPartSites &&
+    return 4 * ml.K[0] * ml.K[1] <= L[0] * L[1] && L[0] <= 2 * kPartSites &&
            ml.K[0] * kNF * (ml.b[1] + 1) <= kPartTasks * kPartThreads &&
            part_smem(L[0], L[1], ml.K[0]) <= 200u * 1024u;
   }
