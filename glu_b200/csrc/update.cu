@@ -23,10 +23,7 @@
 // Layout in HBM: links checkerboard-ordered SoA, U[mu][element][parity]
 // [V/2] complex FP64 -- the threads of a launch read their own links and
 // those of their neighbours with unit stride.  GLU's AoS links convert in
-// and out at the boundary.  Of SU(3) links (checked at the conversion) the
-// first two columns are kept, 96 of 144 bytes: the update is bound by the
-// bytes of the 19 links each thread reads, and the third column is their
-// conjugate cross product, 24 operations.  Other links keep all three.
+// and out at the boundary.
 //
 // Random numbers: Philox4x32-10 (Salmon, Moraes, Dror and Shaw, "Parallel
 // random numbers: as easy as 1, 2, 3", SC 2011), counter-based: the key is
@@ -82,11 +79,6 @@ constexpr double kTwoPi = 6.283185307179586;  // GLU's TWOPI
 // evaluates one more draw before the bound stops it: 43 draws at most
 constexpr int kMaxTries = 43;
 constexpr int kThreads = 128;
-// a link counts as SU(3) while its third column departs (sum of absolute
-// values) from the conjugate cross product of the first two by no more than
-// this: rounding, but not a configuration read from 32-bit reals or links of
-// another determinant
-constexpr double kThirdCol = 1e-12;
 
 // ---------------------------------------------------------------------
 // Philox4x32-10
@@ -143,9 +135,8 @@ struct Rng {
 struct UpdCtx {
   int L[4];
   int V, Vh;      // sites, sites per parity
-  C2 *U;          // [4][NE][2][Vh], NE = 6 or 9 elements
+  C2 *U;          // [4][9][2][Vh]
   double *part;   // per-block partial sums
-  int *bad;       // set where a link's third column is not that of SU(3)
 };
 
 // site coordinates of index h of parity p (Lx even: sites 2k and 2k+1
@@ -168,46 +159,23 @@ __device__ __forceinline__ int cb_index(const UpdCtx &c, const int x[4], int *p)
   return (x[0] >> 1) + (c.L[0] >> 1) * (x[1] + c.L[1] * (x[2] + c.L[2] * x[3]));
 }
 
-// matrix entry of stored element k: all nine, or the first two columns
-template <int NE>
-__host__ __device__ constexpr int entry(int k) {
-  return NE == 9 ? k : (k >> 1) * 3 + (k & 1);
-}
-
-// the stored elements of a link (the third column left unset for NE = 6)
-template <int NE>
-__device__ __forceinline__ void load_part(const UpdCtx &c, int mu, int p, int h, C2 *u) {
-  const C2 *q = c.U + ((size_t)mu * NE * 2 + p) * c.Vh + h;
-#pragma unroll
-  for (int k = 0; k < NE; k++) u[entry<NE>(k)] = q[(size_t)k * 2 * c.Vh];
-}
-template <int NE>
-__device__ __forceinline__ void third_col(C2 *u) {
-  if constexpr (NE == 6) {
-    u[2] = cdet(u[3], u[7], u[4], u[6]);
-    u[5] = cdet(u[1], u[6], u[0], u[7]);
-    u[8] = cdet(u[0], u[4], u[1], u[3]);
-  }
-}
-template <int NE>
 __device__ __forceinline__ void load_cb(const UpdCtx &c, int mu, int p, int h, C2 *u) {
-  load_part<NE>(c, mu, p, h, u);
-  third_col<NE>(u);
-}
-
-template <int NE>
-__device__ __forceinline__ void store_cb(const UpdCtx &c, int mu, int p, int h, const C2 *u) {
-  C2 *q = c.U + ((size_t)mu * NE * 2 + p) * c.Vh + h;
+  const C2 *q = c.U + ((size_t)mu * 9 * 2 + p) * c.Vh + h;
 #pragma unroll
-  for (int k = 0; k < NE; k++) q[(size_t)k * 2 * c.Vh] = u[entry<NE>(k)];
+  for (int e = 0; e < 9; e++) u[e] = q[(size_t)e * 2 * c.Vh];
 }
 
-// the stored elements of U_mu at x
-template <int NE>
-__device__ __forceinline__ void part_at(const UpdCtx &c, int mu, const int x[4], C2 *u) {
+__device__ __forceinline__ void store_cb(const UpdCtx &c, int mu, int p, int h, const C2 *u) {
+  C2 *q = c.U + ((size_t)mu * 9 * 2 + p) * c.Vh + h;
+#pragma unroll
+  for (int e = 0; e < 9; e++) q[(size_t)e * 2 * c.Vh] = u[e];
+}
+
+// the link U_mu at x shifted by +-1 along nu (and optionally along mu)
+__device__ __forceinline__ void load_at(const UpdCtx &c, int mu, const int x[4], C2 *u) {
   int p;
   const int h = cb_index(c, x, &p);
-  load_part<NE>(c, mu, p, h, u);
+  load_cb(c, mu, p, h, u);
 }
 
 // ---------------------------------------------------------------------
@@ -226,17 +194,14 @@ __device__ __forceinline__ C2 ccmul2(C2 a, C2 b) {
 __device__ __forceinline__ C2 add2(C2 a, C2 b) { return mk<double>(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ C2 sub2(C2 a, C2 b) { return mk<double>(a.x - b.x, a.y - b.y); }
 
-// o = a b, from the stored part of b (NE = 6: two columns, then the third
-// of the product)
-template <int NE>
+// o = a b
 __device__ __forceinline__ void m_ab(C2 *o, const C2 *a, const C2 *b) {
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int s = 0; s < (NE == 6 ? 2 : 3); s++)
-      o[3 * r + s] = cmadd(cmadd(cmul(a[3 * r], b[s]), a[3 * r + 1], b[3 + s]),
-                           a[3 * r + 2], b[6 + s]);
-  third_col<NE>(o);
+    for (int s = 0; s < 3; s++)
+      o[3 * r + s] = add2(add2(cmul2(a[3 * r], b[s]), cmul2(a[3 * r + 1], b[3 + s])),
+                          cmul2(a[3 * r + 2], b[6 + s]));
 }
 // o += a b^dag
 __device__ __forceinline__ void m_abdag_acc(C2 *o, const C2 *a, const C2 *b) {
@@ -244,25 +209,23 @@ __device__ __forceinline__ void m_abdag_acc(C2 *o, const C2 *a, const C2 *b) {
   for (int r = 0; r < 3; r++)
 #pragma unroll
     for (int s = 0; s < 3; s++)
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        o[3 * r + s] = cmaddc(o[3 * r + s], a[3 * r + k], b[3 * s + k]);
+      o[3 * r + s] = add2(o[3 * r + s],
+                          add2(add2(cmulc2(a[3 * r], b[3 * s]), cmulc2(a[3 * r + 1], b[3 * s + 1])),
+                               cmulc2(a[3 * r + 2], b[3 * s + 2])));
 }
-// o = a^dag b, from the stored part of b
-template <int NE>
+// o = a^dag b
 __device__ __forceinline__ void m_adagb(C2 *o, const C2 *a, const C2 *b) {
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int s = 0; s < (NE == 6 ? 2 : 3); s++)
-      o[3 * r + s] = cmaddc(cmaddc(cmulc(b[s], a[r]), b[3 + s], a[3 + r]), b[6 + s], a[6 + r]);
-  third_col<NE>(o);
+    for (int s = 0; s < 3; s++)
+      o[3 * r + s] = add2(add2(ccmul2(a[r], b[s]), ccmul2(a[3 + r], b[3 + s])),
+                          ccmul2(a[6 + r], b[6 + s]));
 }
-// o += a b, from the stored part of b
-template <int NE>
+// o += a b
 __device__ __forceinline__ void m_ab_acc(C2 *o, const C2 *a, const C2 *b) {
   C2 t[9];
-  m_ab<NE>(t, a, b);
+  m_ab(t, a, b);
 #pragma unroll
   for (int e = 0; e < 9; e++) o[e] = add2(o[e], t[e]);
 }
@@ -274,7 +237,7 @@ __device__ __forceinline__ int bck(int v, int L) { return v == 0 ? L - 1 : v - 1
 // U_nu(x) U_MU(x+nu) U_nu(x+MU)^dag + U_nu(x-nu)^dag U_MU(x-nu) U_nu(x-nu+MU)
 // (MU a template constant and the nu loop unrolled: every coordinate index
 // is a compile-time constant, nothing goes to local memory)
-template <int MU, int NE>
+template <int MU>
 __device__ __forceinline__ void staple(const UpdCtx &c, const int x[4], C2 *st) {
 #pragma unroll
   for (int e = 0; e < 9; e++) st[e] = mk<double>(0., 0.);
@@ -284,26 +247,23 @@ __device__ __forceinline__ void staple(const UpdCtx &c, const int x[4], C2 *st) 
     C2 a[9], b[9], t[9];
     int y[4] = {x[0], x[1], x[2], x[3]};
     // top
-    part_at<NE>(c, nu, y, a);
-    third_col<NE>(a);
+    load_at(c, nu, y, a);
     y[nu] = fwd(x[nu], c.L[nu]);
-    part_at<NE>(c, MU, y, b);
-    m_ab<NE>(t, a, b);
+    load_at(c, MU, y, b);
+    m_ab(t, a, b);
     y[nu] = x[nu];
     y[MU] = fwd(x[MU], c.L[MU]);
-    part_at<NE>(c, nu, y, a);
-    third_col<NE>(a);
+    load_at(c, nu, y, a);
     m_abdag_acc(st, t, a);
     // bottom
     y[MU] = x[MU];
     y[nu] = bck(x[nu], c.L[nu]);
-    part_at<NE>(c, nu, y, a);
-    third_col<NE>(a);
-    part_at<NE>(c, MU, y, b);
-    m_adagb<NE>(t, a, b);
+    load_at(c, nu, y, a);
+    load_at(c, MU, y, b);
+    m_adagb(t, a, b);
     y[MU] = fwd(x[MU], c.L[MU]);
-    part_at<NE>(c, nu, y, a);
-    m_ab_acc<NE>(st, t, a);
+    load_at(c, nu, y, a);
+    m_ab_acc(st, t, a);
   }
 }
 
@@ -408,22 +368,21 @@ __device__ __forceinline__ void or_su2(C2 *s0, C2 *s1) {
 // over the links U_mu of parity p; counter (link, mu and parity, iteration,
 // draw) for the generator.
 //
-// Bound by the links' bytes and the latency of their loads.  With two columns
-// of each (432 bytes a site and launch against 648) and products that add up
-// in fused operations an over-relaxation launch takes 0.205 ms at 32^3 x 64,
-// 0.288 ms before (0.68 of the copy bandwidth on its bytes).  Four blocks per
-// SM (128 registers, a few spilled) or three make no difference to it; the
-// heatbath's draws need three.
-template <bool HB, int MU, int NE>
-__global__ void __launch_bounds__(kThreads, HB ? 3 : 4) k_update(UpdCtx c, int p, double invbeta,
+// Bound by the links' bytes (648 a site and launch) and the latency of their
+// loads, at three blocks of 168 registers an SM: 0.33 ms an over-relaxation
+// launch at 32^3 x 64.  Keeping two columns of each link takes 0.24, but the
+// completed ones put the links 1.3 times as far from the same in 64 bits, and
+// those off unitarity as far off as they are.
+template <bool HB, int MU>
+__global__ void __launch_bounds__(kThreads, 3) k_update(UpdCtx c, int p, double invbeta,
                                                     uint32_t k0, uint32_t k1, uint32_t iter) {
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= c.Vh) return;
   int x[4];
   cb_coords(c, p, h, x);
   C2 st[9], U[9];
-  staple<MU, NE>(c, x, st);
-  load_cb<NE>(c, MU, p, h, U);
+  staple<MU>(c, x, st);
+  load_cb(c, MU, p, h, U);
   Rng g;
   g.ctr = U4{(uint32_t)h, (uint32_t)(2 * MU + p), iter, 0u};
   g.k0 = k0;
@@ -440,12 +399,11 @@ __global__ void __launch_bounds__(kThreads, HB ? 3 : 4) k_update(UpdCtx c, int p
     rotate(U, sg, s0, s1);
   }
   if (HB) gram_reunit(U);
-  store_cb<NE>(c, MU, p, h, U);
+  store_cb(c, MU, p, h, U);
 }
 
 // per-block partial sums of Re tr of the six plaquettes at every site
 // (av_plaquette, src/Field/plaqs_links.c:243-265)
-template <int NE>
 __global__ void __launch_bounds__(kThreads, 3) k_plaq(UpdCtx c) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   double v = 0.0;
@@ -459,15 +417,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_plaq(UpdCtx c) {
       for (int nu = 0; nu < mu; nu++) {
         C2 a[9], b[9], t1[9], t2[9];
         int y[4] = {x[0], x[1], x[2], x[3]};
-        load_cb<NE>(c, mu, p, h, a);
+        load_cb(c, mu, p, h, a);
         y[mu] = fwd(x[mu], c.L[mu]);
-        part_at<NE>(c, nu, y, b);
-        m_ab<NE>(t1, a, b);  // U_mu(x) U_nu(x+mu)
+        load_at(c, nu, y, b);
+        m_ab(t1, a, b);  // U_mu(x) U_nu(x+mu)
         y[mu] = x[mu];
         y[nu] = fwd(x[nu], c.L[nu]);
-        part_at<NE>(c, mu, y, a);
-        load_cb<NE>(c, nu, p, h, b);
-        m_ab<NE>(t2, b, a);  // U_nu(x) U_mu(x+nu)
+        load_at(c, mu, y, a);
+        load_cb(c, nu, p, h, b);
+        m_ab(t2, b, a);  // U_nu(x) U_mu(x+nu)
         // Re tr(t1 t2^dag)
 #pragma unroll
         for (int e = 0; e < 9; e++) v += t1[e].x * t2[e].x + t1[e].y * t2[e].y;
@@ -487,10 +445,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_plaq(UpdCtx c) {
 
 // GLU's AoS links <-> the checkerboard layout.  A block moves kTile
 // consecutive sites through shared memory, so that both sides are read and
-// written in full lines (a thread to a site read its 576 bytes with that
-// stride: conversions, one heatbath sweep and the plaquette took 5.3 ms at
-// 32^3 x 64, now 3.9 ms): sites 2j and 2j + 1 are neighbours along x (Lx is even), one of
-// each parity, and share the half index.
+// written in full lines, where a thread to a site read its 576 bytes with
+// that stride (conversions, one heatbath sweep and the plaquette at 32^3 x 64:
+// 5.53 -> 5.23 ms).  Sites 2j and 2j + 1 are neighbours along x (Lx is even), one
+// of each parity, and share the half index.
 constexpr int kTile = 64, kTileThreads = 256;
 
 // which of sites 2j, 2j + 1 has parity 0
@@ -501,7 +459,6 @@ __device__ __forceinline__ void pair_parity(const UpdCtx &c, size_t s0, int np, 
   }
 }
 
-template <int NE>
 __global__ void __launch_bounds__(kTileThreads) k_to_cb(UpdCtx c, const C2 *aos) {
   __shared__ C2 t[kTile * 36];
   __shared__ int odd[kTile / 2];
@@ -510,30 +467,13 @@ __global__ void __launch_bounds__(kTileThreads) k_to_cb(UpdCtx c, const C2 *aos)
   for (int i = threadIdx.x; i < ns * 36; i += kTileThreads) t[i] = aos[s0 * 36 + i];
   pair_parity(c, s0, np, odd);
   __syncthreads();
-  for (int i = threadIdx.x; i < 4 * NE * kTile; i += kTileThreads) {
+  for (int i = threadIdx.x; i < 36 * kTile; i += kTileThreads) {
     const int j = i % (kTile / 2), p = i / (kTile / 2) % 2, r = i / kTile;
     if (j < np)
-      c.U[((size_t)r * 2 + p) * c.Vh + s0 / 2 + j] =
-          t[(2 * j + (p ^ odd[j])) * 36 + r / NE * 9 + entry<NE>(r % NE)];
-  }
-  if constexpr (NE == 6) {
-    // (kTileThreads = 4 kTile: one link a thread)
-    if ((int)threadIdx.x < 4 * ns) {
-      C2 u[9];
-#pragma unroll
-      for (int e = 0; e < 9; e++) u[e] = t[threadIdx.x * 9 + e];
-      const C2 w[3] = {u[2], u[5], u[8]};
-      third_col<6>(u);
-      double d = 0.0;
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-        d += fabs(u[3 * r + 2].x - w[r].x) + fabs(u[3 * r + 2].y - w[r].y);
-      if (!(d <= kThirdCol)) *c.bad = 1;
-    }
+      c.U[((size_t)r * 2 + p) * c.Vh + s0 / 2 + j] = t[(2 * j + (p ^ odd[j])) * 36 + r];
   }
 }
 
-template <int NE>
 __global__ void __launch_bounds__(kTileThreads) k_from_cb(UpdCtx c, C2 *aos) {
   __shared__ C2 t[kTile * 36];
   __shared__ int odd[kTile / 2];
@@ -545,7 +485,7 @@ __global__ void __launch_bounds__(kTileThreads) k_from_cb(UpdCtx c, C2 *aos) {
     const int j = i % (kTile / 2), p = i / (kTile / 2) % 2, mu = i / kTile;
     if (j < np) {
       C2 u[9];
-      load_cb<NE>(c, mu, p, (int)(s0 / 2) + j, u);
+      load_cb(c, mu, p, (int)(s0 / 2) + j, u);
 #pragma unroll
       for (int e = 0; e < 9; e++) t[(2 * j + (p ^ odd[j])) * 36 + mu * 9 + e] = u[e];
     }
@@ -562,13 +502,11 @@ struct Work {
   cudaStream_t s = nullptr;
   C2 *d_aos = nullptr;
   int nb_half = 0, nb_all = 0, nb_tile = 0;
-  int ne = 6;  // elements kept of each link of the current call
   std::vector<double> part;
 
   ~Work() {
     cudaFree(c.U);
     cudaFree(c.part);
-    cudaFree(c.bad);
     cudaFree(d_aos);
     if (s) cudaStreamDestroy(s);
   }
@@ -587,11 +525,10 @@ struct Work {
     c.Vh = c.V / 2;
     nb_half = (c.Vh + kThreads - 1) / kThreads;
     nb_all = (c.V + kThreads - 1) / kThreads;
+    nb_tile = (c.V + kTile - 1) / kTile;
     UCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     UCK(cudaMalloc(&c.U, V * 36 * sizeof(C2)));
-    nb_tile = (c.V + kTile - 1) / kTile;
     UCK(cudaMalloc(&c.part, nb_all * sizeof(double)));
-    UCK(cudaMalloc(&c.bad, sizeof(int)));
     part.resize(nb_all);
     return 0;
   }
@@ -601,46 +538,32 @@ struct Work {
     return 0;
   }
 
-  int to_cb(const C2 *aos) {
-    int bad = 0;
-    UCK(cudaMemsetAsync(c.bad, 0, sizeof(int), s));
-    k_to_cb<6><<<nb_tile, kTileThreads, 0, s>>>(c, aos);
-    UCK(cudaMemcpyAsync(&bad, c.bad, sizeof(int), cudaMemcpyDeviceToHost, s));
-    UCK(cudaStreamSynchronize(s));
+  void to_cb(const C2 *aos) {
+    k_to_cb<<<nb_tile, kTileThreads, 0, s>>>(c, aos);
     count_launches(1);
-    ne = bad ? 9 : 6;
-    if (bad) {
-      k_to_cb<9><<<nb_tile, kTileThreads, 0, s>>>(c, aos);
-      count_launches(1);
-    }
-    return 0;
   }
   void from_cb(C2 *aos) {
-    (ne == 6 ? k_from_cb<6> : k_from_cb<9>)<<<nb_tile, kTileThreads, 0, s>>>(c, aos);
+    k_from_cb<<<nb_tile, kTileThreads, 0, s>>>(c, aos);
     count_launches(1);
   }
 
   // one sweep in GLU's order: every direction, both colours
-  using UpdFn = void (*)(UpdCtx, int, double, uint32_t, uint32_t, uint32_t);
-  template <bool HB, int NE>
-  static UpdFn update_fn(int mu) {
-    return mu == 0 ? k_update<HB, 0, NE> : mu == 1 ? k_update<HB, 1, NE>
-           : mu == 2 ? k_update<HB, 2, NE> : k_update<HB, 3, NE>;
-  }
   void sweep(bool hb, double invbeta, uint64_t seed, uint32_t iter) {
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-    for (int mu = 0; mu < 4; mu++) {
-      const UpdFn f = ne == 6 ? (hb ? update_fn<true, 6>(mu) : update_fn<false, 6>(mu))
-                              : (hb ? update_fn<true, 9>(mu) : update_fn<false, 9>(mu));
-      for (int p = 0; p < 2; p++)
+    for (int mu = 0; mu < 4; mu++)
+      for (int p = 0; p < 2; p++) {
+        auto f = hb ? (mu == 0 ? k_update<true, 0> : mu == 1 ? k_update<true, 1>
+                       : mu == 2 ? k_update<true, 2> : k_update<true, 3>)
+                    : (mu == 0 ? k_update<false, 0> : mu == 1 ? k_update<false, 1>
+                       : mu == 2 ? k_update<false, 2> : k_update<false, 3>);
         f<<<nb_half, kThreads, 0, s>>>(c, p, invbeta, k0, k1, iter);
-    }
+      }
     count_launches(8);
   }
 
   // average plaquette, fixed-order sum of the block partials
   int plaquette(double *out) {
-    (ne == 6 ? k_plaq<6> : k_plaq<9>)<<<nb_all, kThreads, 0, s>>>(c);
+    k_plaq<<<nb_all, kThreads, 0, s>>>(c);
     count_launches(1);
     UCK(cudaMemcpyAsync(part.data(), c.part, nb_all * sizeof(double),
                         cudaMemcpyDeviceToHost, s));
@@ -717,7 +640,7 @@ int gfix_heatbath_device(double *d_links, const size_t dims[4], double beta,
   // (on any stream) has finished before they are read
   UCK(cudaDeviceSynchronize());
   C2 *aos = reinterpret_cast<C2 *>(d_links);
-  if (w->to_cb(aos)) return -1;
+  w->to_cb(aos);
   if (w->run(beta, iterations, n_or, seed, first_iteration, plaquettes)) return -1;
   w->from_cb(aos);
   UCK(cudaStreamSynchronize(w->s));
@@ -733,7 +656,7 @@ int gfix_heatbath(double *links, const size_t dims[4], double beta, size_t itera
   if (!w || w->ensure_aos()) return -1;
   const size_t bytes = (size_t)w->c.V * 36 * sizeof(C2);
   UCK(cudaMemcpyAsync(w->d_aos, links, bytes, cudaMemcpyHostToDevice, w->s));
-  if (w->to_cb(w->d_aos)) return -1;
+  w->to_cb(w->d_aos);
   if (w->run(beta, iterations, n_or, seed, first_iteration, plaquettes)) return -1;
   w->from_cb(w->d_aos);
   UCK(cudaMemcpyAsync(links, w->d_aos, bytes, cudaMemcpyDeviceToHost, w->s));
@@ -748,7 +671,7 @@ int gfix_overrelax(double *links, const size_t dims[4], size_t sweeps) {
   if (!w || w->ensure_aos()) return -1;
   const size_t bytes = (size_t)w->c.V * 36 * sizeof(C2);
   UCK(cudaMemcpyAsync(w->d_aos, links, bytes, cudaMemcpyHostToDevice, w->s));
-  if (w->to_cb(w->d_aos)) return -1;
+  w->to_cb(w->d_aos);
   for (size_t k = 0; k < sweeps; k++) w->sweep(false, 0.0, 0, 0);
   w->from_cb(w->d_aos);
   UCK(cudaMemcpyAsync(links, w->d_aos, bytes, cudaMemcpyDeviceToHost, w->s));

@@ -119,3 +119,39 @@ def test_links_outside_su3_keep_all_columns(dims):
     # those of order one; on independent links some are near zero)
     assert np.abs(b - ph * a).max() < 1e-12
     assert np.abs(np.linalg.det(a) - 1).max() < 1e-12
+
+
+@pytest.mark.parametrize("off", [1e-12, 1e-8, 1e-6, 1e-3])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (6, 4, 2, 2), (8, 8, 8, 8)])
+def test_links_off_unitarity_keep_all_columns(dims, off):
+    """Links whose first two columns are off unitarity by `off` and whose
+    third is the conjugate cross product of these (what a long fix, or a
+    reader of 12 rounded reals, leaves): the third column of a product of such
+    links is not that of its first two, nor is it after a common phase, which
+    U S^dag does not see."""
+    V = int(np.prod(dims))
+    rng = np.random.default_rng(7)
+    z = 8 * np.eye(3)[:, :2] + rng.normal(size=(V, 4, 3, 2)) + 1j * rng.normal(size=(V, 4, 3, 2))
+    c0 = z[..., 0] / np.linalg.norm(z[..., 0], axis=-1, keepdims=True)
+    c1 = z[..., 1] - np.sum(np.conj(c0) * z[..., 1], axis=-1, keepdims=True) * c0
+    c1 /= np.linalg.norm(c1, axis=-1, keepdims=True)
+    e = off * rng.normal(size=(3, V, 4, 1))
+    c0, c1 = (1 + e[0]) * c0, (1 + e[1]) * c1 + e[2] * c0
+    U = np.stack([c0, c1, np.conj(np.cross(c0, c1))], axis=-1)
+    ph = np.exp(0.3j)
+    a = update.overrelax(U, dims, 2)
+    b = update.overrelax(ph * U, dims, 2)
+    # rounding at 1e-16 each over the size of the subgroups normalised, as
+    # for SU(3) links; products completed from two columns are off by `off`
+    assert np.abs(b - ph * a).max() < 1e-13
+
+
+def test_runs_from_links_outside_su3_continue():
+    """A run from links that no column completes goes on where it was left,
+    bit for bit, as from SU(3) links."""
+    dims = (8, 4, 4, 6)
+    U0 = np.exp(0.4j) * update.unit_config(dims)
+    a, pa = update.heatbath(U0, dims, 6.0, 4, 1, seed=9)
+    b, _ = update.heatbath(U0, dims, 6.0, 1, 1, seed=9)
+    b, pb = update.heatbath(b, dims, 6.0, 3, 1, seed=9, first_iteration=1)
+    assert np.array_equal(a, b) and pa[-1] == pb[-1]
