@@ -35,6 +35,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <array>
 #include <cmath>
 #include <cstdarg>
@@ -708,13 +709,14 @@ struct CutKey {
 struct MomList {
   std::vector<int> mom;     // 4 per momentum, -pi..pi zone
   std::vector<int2> sites;  // 0..2pi-zone sites of p and -p
-  std::vector<int2> box;    // the same in the box of kept components
+  std::vector<int2> box;    // the same in the box of kept components (partial
+                            // transforms only)
   int b[4] = {0, 0, 0, 0};  // largest |n_mu| of the list
   int K[4] = {1, 1, 1, 1};  // kept components of each axis
   std::vector<C2> phase;    // e^{i p_mu / 2} per momentum and direction
   std::vector<double> pmu;  // 2 sin(p_mu / 2)
   std::vector<double> psq;  // sum_mu pmu^2, 1 below PREC_TOL
-  size_t n() const { return sites.size(); }
+  size_t n() const { return mom.size() / 4; }
 };
 
 // body diagonal d of the hypercube: component mu is +1 where bit mu of d
@@ -763,7 +765,10 @@ static bool cylinder_cjd(const double q[4], double width, double arc) {
   return false;
 }
 
-static int build_list(const int L[4], const gfix_cut_info &ci, MomList &ml) {
+// the kept momenta, 4 integers each, in GLU's order.  Every call of a user asks
+// for these (gfix_cut_veclist) before it measures; what the device needs of them
+// (fill_list, fill_box) is made once and kept with the workspace.
+static std::vector<int> kept_momenta(const int L[4], const gfix_cut_info &ci) {
   int type = ci.type;
   if (ci.dir == GFIX_CUT_NONEXCEPTIONAL) type = GFIX_CUT_PSQ;
   int small = L[0];
@@ -786,7 +791,7 @@ static int build_list(const int L[4], const gfix_cut_info &ci, MomList &ml) {
     lo[mu] = std::max(lo[mu], -b);
     hi[mu] = std::min(hi[mu], b);
   }
-  ml = MomList();
+  std::vector<int> mom;
   int n[4];
   for (n[3] = lo[3]; n[3] <= hi[3]; n[3]++)
     for (n[2] = lo[2]; n[2] <= hi[2]; n[2]++)
@@ -816,40 +821,56 @@ static int build_list(const int L[4], const gfix_cut_info &ci, MomList &ml) {
             ok = psq <= maxm;
           }
           if (!ok) continue;
-          int sp = 0, sn = 0;
-          for (int mu = 3; mu >= 0; mu--) {
-            const int a = n[mu] < 0 ? n[mu] + L[mu] : n[mu];
-            const int b = ((-n[mu]) % L[mu] + L[mu]) % L[mu];
-            sp = sp * L[mu] + a;
-            sn = sn * L[mu] + b;
-          }
-          double ps = 0.;
-          for (int mu = 0; mu < 4; mu++) {
-            ml.mom.push_back(n[mu]);
-            const double cache = 0.5 * n[mu] * tw[mu];
-            const double p = 2.0 * std::sin(cache);
-            ml.phase.push_back(mk<double>(std::cos(cache), 0.5 * p));
-            const double m = 2.0 * std::sin(n[mu] * tw[mu] * 0.5);
-            ml.pmu.push_back(m);
-            ps += m * m;
-          }
-          ml.psq.push_back(ps < kPrecTol ? 1.0 : ps);
-          ml.sites.push_back(make_int2(sp, sn));
+          mom.insert(mom.end(), n, n + 4);
         }
-  for (size_t i = 0; i < ml.n(); i++)
-    for (int mu = 0; mu < 4; mu++) ml.b[mu] = std::max(ml.b[mu], std::abs(ml.mom[i * 4 + mu]));
+  return mom;
+}
+
+// sites, phases and lattice momenta of ml.mom, and the components its axes keep
+static void fill_list(const int L[4], MomList &ml) {
+  double tw[4];
+  for (int mu = 0; mu < 4; mu++) tw[mu] = kTwoPi / (double)L[mu];
+  ml.sites.reserve(ml.n());
+  ml.phase.reserve(4 * ml.n());
+  ml.pmu.reserve(4 * ml.n());
+  ml.psq.reserve(ml.n());
+  for (size_t i = 0; i < ml.n(); i++) {
+    const int *n = &ml.mom[4 * i];
+    int sp = 0, sn = 0;
+    double ps = 0.;
+    for (int mu = 3; mu >= 0; mu--) {
+      sp = sp * L[mu] + (n[mu] < 0 ? n[mu] + L[mu] : n[mu]);
+      sn = sn * L[mu] + (n[mu] > 0 ? L[mu] - n[mu] : -n[mu]);
+    }
+    for (int mu = 0; mu < 4; mu++) {
+      const double cache = 0.5 * n[mu] * tw[mu];
+      const double p = 2.0 * std::sin(cache);
+      ml.phase.push_back(mk<double>(std::cos(cache), 0.5 * p));
+      const double m = 2.0 * std::sin(n[mu] * tw[mu] * 0.5);
+      ml.pmu.push_back(m);
+      ps += m * m;
+      ml.b[mu] = std::max(ml.b[mu], std::abs(n[mu]));
+    }
+    ml.psq.push_back(ps < kPrecTol ? 1.0 : ps);
+    ml.sites.push_back(make_int2(sp, sn));
+  }
   for (int mu = 0; mu < 4; mu++) ml.K[mu] = std::min(L[mu], 2 * ml.b[mu] + 1);
+}
+
+// places of p and -p in the box of kept components: n from the front of its
+// axis, -n from the back (n = -L/2, which is L/2, from the front where the
+// axis keeps all of its components)
+static void fill_box(const int L[4], MomList &ml) {
+  ml.box.reserve(ml.n());
   for (size_t i = 0; i < ml.n(); i++) {
     int s[2] = {0, 0};
     for (int mu = 3; mu >= 0; mu--)
       for (int k = 0; k < 2; k++) {
         const int m = k ? -ml.mom[i * 4 + mu] : ml.mom[i * 4 + mu];
-        const int r = (m % L[mu] + L[mu]) % L[mu];  // residue, then its place
-        s[k] = s[k] * ml.K[mu] + (r <= ml.b[mu] ? r : ml.K[mu] - (L[mu] - r));
+        s[k] = s[k] * ml.K[mu] + (m >= 0 ? m : 2 * m == -L[mu] ? -m : ml.K[mu] + m);
       }
     ml.box.push_back(make_int2(s[0], s[1]));
   }
-  return 0;
 }
 
 // ---------------------------------------------------------------------
@@ -1019,7 +1040,9 @@ struct Work {
     auto it = lists.find(k);
     if (it != lists.end()) return &it->second;
     MomList ml;
-    if (build_list(L, ci, ml)) return nullptr;
+    ml.mom = kept_momenta(L, ci);
+    fill_list(L, ml);
+    if (partial(ml)) fill_box(L, ml);
     return &lists.emplace(k, std::move(ml)).first->second;
   }
 
@@ -1343,12 +1366,10 @@ long gfix_cut_veclist(const size_t dims[4], const gfix_cut_info *ci, int32_t *mo
     if (dims[i] < 2 || dims[i] > 4096) return cfail("extent %zu outside 2..4096", dims[i]);
     L[i] = (int)dims[i];
   }
-  MomList ml;
-  if (build_list(L, *ci, ml)) return -1;
-  if (mom)
-    for (size_t i = 0; i < ml.n() && i < cap; i++)
-      for (int mu = 0; mu < 4; mu++) mom[i * 4 + mu] = ml.mom[i * 4 + mu];
-  return (long)ml.n();
+  const std::vector<int> kept = kept_momenta(L, *ci);
+  const size_t n = kept.size() / 4;
+  if (mom) std::copy_n(kept.begin(), 4 * std::min(n, cap), mom);
+  return (long)n;
 }
 
 int gfix_cuts_measure_device(const double *d_links, const size_t dims[4],
