@@ -47,6 +47,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/glu_gfix.h"
@@ -404,6 +405,35 @@ __device__ __forceinline__ void pair_add(C2 f, C2 w, C2 *p, C2 *q) {
   q->x = fma(f.x, -w.y, q->x);
   q->y = fma(f.y, -w.y, q->y);
 }
+// p and q of n elements, k ld apart and k step of the table's len on; in blocks
+// of eight, whose sums are added: the rounding of a sum of N terms grows as
+// sqrt(N) where a transform's grows as its stages.  With one chain for each axis
+// the fields at 32^3 x 64 were 6.9e-16 from their values (5.7e-16 by the full
+// transforms; 5.9e-16 now, 4.3e-16 with the factors of Work::init)
+__device__ __forceinline__ void pair_sum(const C2 *f, size_t ld, int n, const C2 *tw, int step,
+                                         int len, C2 *p, C2 *q) {
+  constexpr int kB = 8;
+  C2 P = mk<double>(0., 0.), Q = P;
+  int w = 0, k = 0;
+  auto block = [&](auto trips) {
+    C2 a = mk<double>(0., 0.), b = a;
+#pragma unroll
+    for (int j = 0; j < decltype(trips)::value; j++) {
+      pair_add(f[(size_t)(k + j) * ld], tw[w], &a, &b);
+      w += step;
+      w -= w >= len ? len : 0;
+    }
+    P = cadd(P, a);
+    Q = cadd(Q, b);
+    k += decltype(trips)::value;
+  };
+#pragma unroll 1
+  while (k + kB <= n) block(std::integral_constant<int, kB>{});
+#pragma unroll 1
+  while (k < n) block(std::integral_constant<int, 1>{});
+  *p = P;
+  *q = Q;
+}
 // sum f e^{+i n theta} and sum f e^{-i n theta}
 __device__ __forceinline__ C2 pair_pos(C2 p, C2 q) { return mk<double>(p.x - q.y, p.y + q.x); }
 __device__ __forceinline__ C2 pair_neg(C2 p, C2 q) { return mk<double>(p.x + q.y, p.y - q.x); }
@@ -448,15 +478,8 @@ __global__ void __launch_bounds__(kPartThreads) k_cut_pxy(PartCtx c) {
     // x: field fastest, then the row, then the pair
     for (int o = threadIdx.x; o < rows * kNF * nx; o += kPartThreads) {
       const int f = o % kNF, r = o / kNF % rows, n = o / kNF / rows;
-      const C2 *a = A + (size_t)r * Lx * kNF + f;
-      C2 p = mk<double>(0., 0.), q = p;
-      int w = 0;
-#pragma unroll 4
-      for (int x = 0; x < Lx; x++) {
-        pair_add(a[x * kNF], twx[w], &p, &q);
-        w += n;
-        w -= w >= Lx ? Lx : 0;
-      }
+      C2 p, q;
+      pair_sum(A + (size_t)r * Lx * kNF + f, kNF, Lx, twx, n, Lx, &p, &q);
       C2 *d = X + (size_t)r * Q + f;
       d[n * kNF] = pair_pos(p, q);
       if (n && 2 * n != Lx) d[(Kx - n) * kNF] = pair_neg(p, q);
@@ -469,11 +492,14 @@ __global__ void __launch_bounds__(kPartThreads) k_cut_pxy(PartCtx c) {
       if (o < Q * ny) {
         const int n = o / Q, col = o - n * Q;
         int w = (int)((long long)n * y0 % Ly);
+        C2 a = mk<double>(0., 0.), b = a;
         for (int r = 0; r < rows; r++) {
-          pair_add(X[(size_t)r * Q + col], twy[w], &P[k], &S[k]);
+          pair_add(X[(size_t)r * Q + col], twy[w], &a, &b);
           w += n;
           w -= w >= Ly ? Ly : 0;
         }
+        P[k] = cadd(P[k], a);
+        S[k] = cadd(S[k], b);
       }
     }
     // (the next chunk's x sums follow a barrier, after which X is free)
@@ -496,15 +522,8 @@ __global__ void __launch_bounds__(128) k_cut_part(const C2 *in, C2 *out, const C
                                                   int K, int C) {
   const int col = blockIdx.x * blockDim.x + threadIdx.x, n = blockIdx.z;
   if (col >= C) return;
-  const C2 *a = in + (size_t)blockIdx.y * len * C + col;
-  C2 p = mk<double>(0., 0.), q = p;
-  int w = 0;
-#pragma unroll 8
-  for (int k = 0; k < len; k++) {
-    pair_add(a[(size_t)k * C], tw[w], &p, &q);
-    w += n;
-    w -= w >= len ? len : 0;
-  }
+  C2 p, q;
+  pair_sum(in + (size_t)blockIdx.y * len * C + col, C, len, tw, n, len, &p, &q);
   C2 *d = out + (size_t)blockIdx.y * K * C + col;
   d[(size_t)n * C] = pair_pos(p, q);
   if (n && 2 * n != len) d[(size_t)(K - n) * C] = pair_neg(p, q);
@@ -964,8 +983,10 @@ struct Work {
     for (int a = 0; a < 4; a++) {
       c.ax[a].tw_off = (int)tw.size();
       for (int k = 0; k < L[a]; k++) {
-        const double ang = 6.283185307179586476925286766559 * k / L[a];
-        tw.push_back(mk<double>(std::cos(ang), -std::sin(ang)));
+        // (in 64-bit mantissas: rounding the angle in 53 alone would put the
+        // factors up to 5e-16 off)
+        const long double ang = 6.283185307179586476925286766559L * k / L[a];
+        tw.push_back(mk<double>((double)std::cos(ang), -(double)std::sin(ang)));
       }
     }
     CCK(cudaMalloc(&d_tw, tw.size() * sizeof(C2)));
