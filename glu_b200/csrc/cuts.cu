@@ -967,7 +967,7 @@ struct Work {
     // compile-time passes where the extents have them
     if (!odd) {
       const size_t sm4 = (4 * (size_t)(L[0] + 1) * L[1] + L[0] + L[1]) * sizeof(C2);
-      if (xy4_ct(L[0], L[1], false) && sm4 <= 200u * 1024u) {
+      if (xy4_ct(L[0], L[1], false) && sm4 <= kSmemMax) {
         xy4 = true;
         xy_fn[0] = xy4_ct(L[0], L[1], false);
         xy_fn[1] = xy4_ct(L[0], L[1], true);
@@ -1013,7 +1013,7 @@ struct Work {
     for (const auto &cd : cands) {
       const int bw = cd.first;
       const size_t sm = ((size_t)(L[2] * bw + zt_pad(bw)) * L[3] + L[2] + L[3]) * sizeof(C2);
-      if (sm > 200u * 1024u || attr(cd.second, sm)) continue;
+      if (sm > kSmemMax || attr(cd.second)) continue;
       CutCtx cc = c;
       cc.zt_b = bw;
       const int bd = ct_threads(bw * L[2] * L[3]);
@@ -1039,20 +1039,26 @@ struct Work {
     return 0;
   }
 
+  // the shared-memory limit is the function's, not a launch's or a workspace's:
+  // every one sets the same, the most that any lattice takes, so that no lattice
+  // lowers it under the launches of another, in this thread or the next
+  static constexpr size_t kSmemMax = 200 * 1024;
   template <typename K>
-  int attr(K k, size_t sm) {
-    CCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  int attr(K k) {
+    CCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     return 0;
   }
   int set_attrs() {
-    if (attr(k_cut_xy<8, false, true>, sm_xy) || attr(k_cut_xy<16, false, true>, sm_xy) ||
-        attr(k_cut_xy<16, true, true>, sm_xy) || attr(k_cut_xy<8, false, false>, sm_xy) ||
-        attr(k_cut_xy<16, false, false>, sm_xy) || attr(k_cut_xy<16, true, false>, sm_xy) ||
-        attr(k_cut_zt<8, false>, sm_zt) || attr(k_cut_zt<16, false>, sm_zt) ||
-        attr(k_cut_zt<16, true>, sm_zt))
+    if (attr(k_cut_xy<8, false, true>) || attr(k_cut_xy<16, false, true>) ||
+        attr(k_cut_xy<16, true, true>) || attr(k_cut_xy<8, false, false>) ||
+        attr(k_cut_xy<16, false, false>) || attr(k_cut_xy<16, true, false>) ||
+        attr(k_cut_zt<8, false>) || attr(k_cut_zt<16, false>) || attr(k_cut_zt<16, true>) ||
+        attr(k_cut_pxy<false, 1>) || attr(k_cut_pxy<false, 3>) ||
+        attr(k_cut_pxy<false, kPartTasks>) || attr(k_cut_pxy<true, 1>) ||
+        attr(k_cut_pxy<true, 3>) || attr(k_cut_pxy<true, kPartTasks>))
       return -1;
     for (CutFn f : xy_fn)
-      if (f && attr(f, sm_xy)) return -1;
+      if (f && attr(f)) return -1;
     return 0;
   }
 
@@ -1076,7 +1082,7 @@ struct Work {
   bool partial(const MomList &ml) const {
     return 4 * ml.K[0] * ml.K[1] <= L[0] * L[1] && L[0] <= 2 * kPartSites &&
            ml.K[0] * kNF * (ml.b[1] + 1) <= kPartTasks * kPartThreads &&
-           part_smem(L[0], L[1], ml.K[0]) <= 200u * 1024u;
+           part_smem(L[0], L[1], ml.K[0]) <= kSmemMax;
   }
 
   int upload(const MomList *ml) {
@@ -1147,18 +1153,16 @@ struct Work {
     return p;
   }
   template <bool LOG>
-  int part_pxy(const PartCtx &p) {
+  void part_pxy(const PartCtx &p) {
     const int tasks = (p.K[0] * kNF * (p.b[1] + 1) + kPartThreads - 1) / kPartThreads;
     auto f = tasks <= 1 ? k_cut_pxy<LOG, 1> : tasks <= 3 ? k_cut_pxy<LOG, 3>
                                                          : k_cut_pxy<LOG, kPartTasks>;
     const size_t sm = part_smem(L[0], L[1], p.K[0]);
-    if (attr(f, sm)) return -1;
     f<<<L[2] * L[3], kPartThreads, sm, s>>>(p);
-    return 0;
   }
-  int transform_part(bool log, cudaEvent_t mid) {
+  void transform_part(bool log, cudaEvent_t mid) {
     const PartCtx p = part_ctx();
-    if (log ? part_pxy<true>(p) : part_pxy<false>(p)) return -1;
+    log ? part_pxy<true>(p) : part_pxy<false>(p);
     if (mid) cudaEventRecord(mid, s);
     const int C = kNF * p.K[0] * p.K[1], Cz = C * p.K[2];
     k_cut_part<<<dim3((C + 127) / 128, L[3], p.b[2] + 1), 128, 0, s>>>(
@@ -1166,12 +1170,11 @@ struct Work {
     k_cut_part<<<dim3((Cz + 127) / 128, 1, p.b[3] + 1), 128, 0, s>>>(
         p.F2, p.F3, d_tw + p.tw_off[3], L[3], p.K[3], Cz);
     count_launches(3);
-    return 0;
   }
 
   // the transforms of the Lie fields (definition def) of c.links into
   // d_F; `mid` (may be null) is recorded between the xy and the zt pass
-  int transform(int def, cudaEvent_t mid = nullptr) {
+  void transform(int def, cudaEvent_t mid = nullptr) {
     const bool log = def == GFIX_FIELD_LOG;
     if (part) return transform_part(log, mid);
     const dim3 gxy(xy4 ? 4 : kNF, L[2] * L[3]);
@@ -1201,7 +1204,6 @@ struct Work {
     else
       k_cut_zt<16, false><<<gzt, bd_zt, sm_zt, s>>>(c);
     count_launches(2);
-    return 0;
   }
 
   Norms norms() const {
@@ -1298,7 +1300,7 @@ static int run(Work *w, const gfix_cut_info *ci, size_t nmom, double *out0,
   if (nmom != ml->n())
     return cfail("%zu momenta given, the cut keeps %zu", nmom, ml->n());
   if (w->upload(ml)) return -1;
-  if (w->transform(ci->definition)) return -1;
+  w->transform(ci->definition);
   w->measure(ci->dir);
   CCK(cudaGetLastError());
   return w->fetch(ci->dir, out0, out1, perr);
@@ -1453,7 +1455,7 @@ int gfix_profile_cuts(const double *d_links, const size_t dims[4], const gfix_cu
   float acc[3] = {0, 0, 0};
   for (int r = 0; r < reps + 1; r++) {
     CCK(cudaEventRecord(ev[0], w->s));
-    if (w->transform(ci->definition, ev[1])) return -1;
+    w->transform(ci->definition, ev[1]);
     CCK(cudaEventRecord(ev[2], w->s));
     w->measure(ci->dir);
     CCK(cudaEventRecord(ev[3], w->s));

@@ -254,3 +254,26 @@ def test_fields_to_rounding(dims, maxmom):
     # 0.4e-16 in the mean for each, as much again for the factors and fields
     assert err < 4.2e-16, err
     assert len(n) > 1
+
+
+def test_lattices_leave_each_other_their_shared_memory():
+    """The limit of a pass's shared memory is the function's: a small lattice
+    must not lower it under a large one met before, nor one thread's under
+    another's."""
+    from concurrent.futures import ThreadPoolExecutor
+    info = cuts.CutInfo("FIELDS", "SPHERICAL_CUT", "LINEAR", 1)
+    large, small = (60, 60, 2, 2), (6, 6, 4, 4)  # generic passes of 60 and 1 KB
+    U = {d: _links(d) for d in (large, small)}
+    first = {d: cuts.measure(U[d], d, info) for d in (large, small)}
+    again = cuts.measure(U[large], large, info)
+    assert np.array_equal(first[large]["fields"], again["fields"])
+    # partial transforms, whose limits differ with the extents
+    dims = [(48, 16, 8, 8), (16, 16, 8, 8), (30, 30, 6, 6), (12, 12, 6, 6)]
+    L = {d: _links(d) for d in dims}
+    ref = {d: cuts.measure(L[d], d, info)["fields"] for d in dims}
+
+    def repeat(d):
+        return all(np.array_equal(cuts.measure(L[d], d, info)["fields"], ref[d])
+                   for _ in range(25))
+    with ThreadPoolExecutor(len(dims)) as ex:
+        assert all(ex.map(repeat, dims))
