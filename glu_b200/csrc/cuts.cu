@@ -48,6 +48,7 @@
 #include <string>
 #include <tuple>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/glu_gfix.h"
@@ -1013,7 +1014,7 @@ struct Work {
     for (const auto &cd : cands) {
       const int bw = cd.first;
       const size_t sm = ((size_t)(L[2] * bw + zt_pad(bw)) * L[3] + L[2] + L[3]) * sizeof(C2);
-      if (sm > kSmemMax || attr(cd.second)) continue;
+      if (sm > kSmemMax || attr(cd.second, sm)) continue;
       CutCtx cc = c;
       cc.zt_b = bw;
       const int bd = ct_threads(bw * L[2] * L[3]);
@@ -1039,26 +1040,33 @@ struct Work {
     return 0;
   }
 
-  // the shared-memory limit is the function's, not a launch's or a workspace's:
-  // every one sets the same, the most that any lattice takes, so that no lattice
-  // lowers it under the launches of another, in this thread or the next
+  // The shared-memory limit is the function's, not a launch's or a workspace's:
+  // it is only ever raised, so that no lattice lowers it under the launches of
+  // another, in this thread or the next.  (The largest at once costs the generic
+  // passes, whose spills live in the L1 that it leaves, up to 18%.)
   static constexpr size_t kSmemMax = 200 * 1024;
   template <typename K>
-  int attr(K k) {
-    CCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
+  static int attr(K k, size_t sm) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limit;
+    int dev = 0;
+    CCK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    size_t &cur = limit[{dev, (const void *)k}];
+    if (sm <= cur) return 0;
+    CCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    cur = sm;
     return 0;
   }
   int set_attrs() {
-    if (attr(k_cut_xy<8, false, true>) || attr(k_cut_xy<16, false, true>) ||
-        attr(k_cut_xy<16, true, true>) || attr(k_cut_xy<8, false, false>) ||
-        attr(k_cut_xy<16, false, false>) || attr(k_cut_xy<16, true, false>) ||
-        attr(k_cut_zt<8, false>) || attr(k_cut_zt<16, false>) || attr(k_cut_zt<16, true>) ||
-        attr(k_cut_pxy<false, 1>) || attr(k_cut_pxy<false, 3>) ||
-        attr(k_cut_pxy<false, kPartTasks>) || attr(k_cut_pxy<true, 1>) ||
-        attr(k_cut_pxy<true, 3>) || attr(k_cut_pxy<true, kPartTasks>))
+    if (attr(k_cut_xy<8, false, true>, sm_xy) || attr(k_cut_xy<16, false, true>, sm_xy) ||
+        attr(k_cut_xy<16, true, true>, sm_xy) || attr(k_cut_xy<8, false, false>, sm_xy) ||
+        attr(k_cut_xy<16, false, false>, sm_xy) || attr(k_cut_xy<16, true, false>, sm_xy) ||
+        attr(k_cut_zt<8, false>, sm_zt) || attr(k_cut_zt<16, false>, sm_zt) ||
+        attr(k_cut_zt<16, true>, sm_zt))
       return -1;
     for (CutFn f : xy_fn)
-      if (f && attr(f)) return -1;
+      if (f && attr(f, sm_xy)) return -1;
     return 0;
   }
 
@@ -1153,16 +1161,18 @@ struct Work {
     return p;
   }
   template <bool LOG>
-  void part_pxy(const PartCtx &p) {
+  int part_pxy(const PartCtx &p) {
     const int tasks = (p.K[0] * kNF * (p.b[1] + 1) + kPartThreads - 1) / kPartThreads;
     auto f = tasks <= 1 ? k_cut_pxy<LOG, 1> : tasks <= 3 ? k_cut_pxy<LOG, 3>
                                                          : k_cut_pxy<LOG, kPartTasks>;
     const size_t sm = part_smem(L[0], L[1], p.K[0]);
+    if (attr(f, sm)) return -1;
     f<<<L[2] * L[3], kPartThreads, sm, s>>>(p);
+    return 0;
   }
-  void transform_part(bool log, cudaEvent_t mid) {
+  int transform_part(bool log, cudaEvent_t mid) {
     const PartCtx p = part_ctx();
-    log ? part_pxy<true>(p) : part_pxy<false>(p);
+    if (log ? part_pxy<true>(p) : part_pxy<false>(p)) return -1;
     if (mid) cudaEventRecord(mid, s);
     const int C = kNF * p.K[0] * p.K[1], Cz = C * p.K[2];
     k_cut_part<<<dim3((C + 127) / 128, L[3], p.b[2] + 1), 128, 0, s>>>(
@@ -1170,11 +1180,12 @@ struct Work {
     k_cut_part<<<dim3((Cz + 127) / 128, 1, p.b[3] + 1), 128, 0, s>>>(
         p.F2, p.F3, d_tw + p.tw_off[3], L[3], p.K[3], Cz);
     count_launches(3);
+    return 0;
   }
 
   // the transforms of the Lie fields (definition def) of c.links into
   // d_F; `mid` (may be null) is recorded between the xy and the zt pass
-  void transform(int def, cudaEvent_t mid = nullptr) {
+  int transform(int def, cudaEvent_t mid = nullptr) {
     const bool log = def == GFIX_FIELD_LOG;
     if (part) return transform_part(log, mid);
     const dim3 gxy(xy4 ? 4 : kNF, L[2] * L[3]);
@@ -1204,6 +1215,7 @@ struct Work {
     else
       k_cut_zt<16, false><<<gzt, bd_zt, sm_zt, s>>>(c);
     count_launches(2);
+    return 0;
   }
 
   Norms norms() const {
@@ -1300,7 +1312,7 @@ static int run(Work *w, const gfix_cut_info *ci, size_t nmom, double *out0,
   if (nmom != ml->n())
     return cfail("%zu momenta given, the cut keeps %zu", nmom, ml->n());
   if (w->upload(ml)) return -1;
-  w->transform(ci->definition);
+  if (w->transform(ci->definition)) return -1;
   w->measure(ci->dir);
   CCK(cudaGetLastError());
   return w->fetch(ci->dir, out0, out1, perr);
@@ -1455,7 +1467,7 @@ int gfix_profile_cuts(const double *d_links, const size_t dims[4], const gfix_cu
   float acc[3] = {0, 0, 0};
   for (int r = 0; r < reps + 1; r++) {
     CCK(cudaEventRecord(ev[0], w->s));
-    w->transform(ci->definition, ev[1]);
+    if (w->transform(ci->definition, ev[1])) return -1;
     CCK(cudaEventRecord(ev[2], w->s));
     w->measure(ci->dir);
     CCK(cudaEventRecord(ev[3], w->s));
