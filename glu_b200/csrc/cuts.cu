@@ -905,7 +905,7 @@ struct Work {
      *d_phase = nullptr;
   double *d_pmu = nullptr, *d_psq = nullptr, *d_err = nullptr, *d_o0 = nullptr,
          *d_o1 = nullptr;
-  int2 *d_sites = nullptr;
+  int2 *d_sites = nullptr, *d_box = nullptr;
   size_t cap = 0;  // momenta the list buffers hold
   int pt_xy = 8, pt_zt = 8, bd_xy = 128, bd_zt = 128;
   size_t sm_xy = 0, sm_zt = 0;
@@ -915,7 +915,7 @@ struct Work {
   bool xy4 = false;  // xy_fn are k_cut_xy4_ct (the Lie fields computed inside)
   std::map<CutKey, MomList> lists;
   const MomList *cur = nullptr;  // list on the device
-  bool part = false;             // its momenta by partial transforms
+  bool part = false;             // d_F holds their partial transforms
 
   ~Work() {
     cudaFree(d_links);
@@ -929,6 +929,7 @@ struct Work {
     cudaFree(d_o0);
     cudaFree(d_o1);
     cudaFree(d_sites);
+    cudaFree(d_box);
     if (s) cudaStreamDestroy(s);
   }
 
@@ -1077,20 +1078,42 @@ struct Work {
     MomList ml;
     ml.mom = kept_momenta(L, ci);
     fill_list(L, ml);
-    if (partial(ml)) fill_box(L, ml);
+    if (can_part(ml)) fill_box(L, ml);
     return &lists.emplace(k, std::move(ml)).first->second;
   }
 
   // Partial transforms serve a list whose kept components are at most a
   // quarter of an xy plane (the fields they leave then fit in d_F, three
-  // times): both passes take 0.197 against 0.459 ms with 81 of 400 components
-  // (20^3 x 40), 0.858 against 1.274 ms with 81 of 1024 (32^3 x 64), but 0.090
-  // against 0.084 ms with 81 of 256 (16^3 x 32).  Their rows must be short
-  // enough for a chunk of them in shared memory.
-  bool partial(const MomList &ml) const {
+  // times) and whose rows are short enough for a chunk of them in shared memory,
+  // where they are faster.  Their first pass gives a block to each plane, so few
+  // planes leave SMs idle, with logarithms above all, which take a block longer
+  // than its sums.  Both passes in ms, partial against full:
+  //   generic full passes: where a plane has at most 36 sites for each of the
+  //     planes (32^2 of 25 0.067 against 0.050, of 30 0.067 each, of 49 0.058
+  //     against 0.095; 36^2 of 36 0.080 against 0.144), with logarithms 14, and
+  //     a sixth of them kept (24^2 of 30 0.075 against 0.065; of 49 0.087 against
+  //     0.076 for 121 components, 0.074 against 0.075 for 49; 25^2 of 49 0.080
+  //     against 0.164);
+  //   a compiled xy pass: from 40 planes (24^2 of 36 0.042 against 0.043, of 49
+  //     0.038 against 0.068), with logarithms from 80 (24^2 of 72 0.082 against
+  //     0.066, of 80 0.073 against 0.109);
+  //   both passes compiled: from more planes than SMs and 16^2 sites (24^2 of 128
+  //     0.050 against 0.044, of 256 0.067 against 0.074; 8^2 of 512 0.030 against
+  //     0.026), with logarithms for an eighth of the plane (24^2 of 512 0.170
+  //     against 0.174 for 49 components, 0.208 for 121).
+  bool can_part(const MomList &ml) const {
     return 4 * ml.K[0] * ml.K[1] <= L[0] * L[1] && L[0] <= 2 * kPartSites &&
            ml.K[0] * kNF * (ml.b[1] + 1) <= kPartTasks * kPartThreads &&
            part_smem(L[0], L[1], ml.K[0]) <= kSmemMax;
+  }
+  bool partial(const MomList &ml, bool log) const {
+    if (!can_part(ml)) return false;
+    const int plane = L[0] * L[1], planes = L[2] * L[3], kept = ml.K[0] * ml.K[1];
+    constexpr int kSms = 148;
+    if (plane > (log ? 14 : 36) * planes || (log && 6 * kept > plane)) return false;
+    if (!xy_fn[log]) return true;
+    if (!zt_fn) return planes >= (log ? 80 : 40);
+    return planes > kSms && (log ? 8 * kept <= plane : plane >= 256);
   }
 
   int upload(const MomList *ml) {
@@ -1105,9 +1128,10 @@ struct Work {
       cudaFree(d_o0);
       cudaFree(d_o1);
       cudaFree(d_sites);
+      cudaFree(d_box);
       d_G = d_phase = nullptr;
       d_pmu = d_psq = d_err = d_o0 = d_o1 = nullptr;
-      d_sites = nullptr;
+      d_sites = d_box = nullptr;
       cap = 0;
       CCK(cudaMalloc(&d_G, n * 36 * sizeof(C2)));
       CCK(cudaMalloc(&d_phase, n * 4 * sizeof(C2)));
@@ -1117,10 +1141,10 @@ struct Work {
       CCK(cudaMalloc(&d_o0, n * sizeof(double)));
       CCK(cudaMalloc(&d_o1, n * sizeof(double)));
       CCK(cudaMalloc(&d_sites, n * sizeof(int2)));
+      CCK(cudaMalloc(&d_box, n * sizeof(int2)));
       cap = n;
     }
     cur = nullptr;
-    const bool pt = partial(*ml);
     if (ml->n()) {
       CCK(cudaMemcpyAsync(d_phase, ml->phase.data(), ml->n() * 4 * sizeof(C2),
                           cudaMemcpyHostToDevice, s));
@@ -1128,12 +1152,14 @@ struct Work {
                           cudaMemcpyHostToDevice, s));
       CCK(cudaMemcpyAsync(d_psq, ml->psq.data(), ml->n() * sizeof(double),
                           cudaMemcpyHostToDevice, s));
-      CCK(cudaMemcpyAsync(d_sites, (pt ? ml->box : ml->sites).data(), ml->n() * sizeof(int2),
+      CCK(cudaMemcpyAsync(d_sites, ml->sites.data(), ml->n() * sizeof(int2),
                           cudaMemcpyHostToDevice, s));
+      if (!ml->box.empty())
+        CCK(cudaMemcpyAsync(d_box, ml->box.data(), ml->n() * sizeof(int2),
+                            cudaMemcpyHostToDevice, s));
     }
     CCK(cudaStreamSynchronize(s));
     cur = ml;
-    part = pt;
     return 0;
   }
 
@@ -1187,6 +1213,7 @@ struct Work {
   // d_F; `mid` (may be null) is recorded between the xy and the zt pass
   int transform(int def, cudaEvent_t mid = nullptr) {
     const bool log = def == GFIX_FIELD_LOG;
+    part = partial(*cur, log);
     if (part) return transform_part(log, mid);
     const dim3 gxy(xy4 ? 4 : kNF, L[2] * L[3]);
     if (log && !xy4) {
@@ -1230,7 +1257,7 @@ struct Work {
     if (n == 0) return;
     const int nb = (n + 127) / 128;
     if (part)
-      k_cut_gather<<<nb, 128, 0, s>>>(part_ctx().F3, kNF, 1, 1, n, d_sites, d_phase, d_pmu, d_G,
+      k_cut_gather<<<nb, 128, 0, s>>>(part_ctx().F3, kNF, 1, 1, n, d_box, d_phase, d_pmu, d_G,
                                       d_err);
     else
       k_cut_gather<<<nb, 128, 0, s>>>(d_F, 1, V, 0, n, d_sites, d_phase, d_pmu, d_G, d_err);

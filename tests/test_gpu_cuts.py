@@ -277,3 +277,21 @@ def test_lattices_leave_each_other_their_shared_memory():
                    for _ in range(25))
     with ThreadPoolExecutor(len(dims)) as ex:
         assert all(ex.map(repeat, dims))
+
+
+@pytest.mark.parametrize("dims,maxmom", [((24, 24, 6, 12), 1), ((20, 20, 5, 5), 1),
+                                         ((16, 16, 16, 16), 2), ((28, 28, 6, 6), 1)])
+def test_definitions_take_turns_on_one_list(dims, maxmom):
+    """Logarithms may take the full transforms of a list whose linear fields
+    take the partial ones: each reads its own places of the same list."""
+    U = _links(dims)
+    kw = dict(cuttype="FIELDS", mom_cut="SPHERICAL_CUT")
+    every = {f: cuts.measure(U, dims, cuts.CutInfo(field_definition=f, maxmom=max(dims) ** 2, **kw))
+             for f in ("LINEAR", "LOGARITHMIC")}
+    at = {tuple(m): i for i, m in enumerate(every["LINEAR"]["mom"])}
+    for f in ("LINEAR", "LOGARITHMIC", "LINEAR", "LOGARITHMIC"):
+        r = cuts.measure(U, dims, cuts.CutInfo(field_definition=f, maxmom=maxmom, **kw))
+        w = every[f]["fields"][[at[tuple(m)] for m in r["mom"]]]
+        # sums of V terms of order one
+        assert np.abs(r["fields"] - w).max() < 1e-14 * np.prod(dims)
+        assert np.abs(w).max() > 1.0
