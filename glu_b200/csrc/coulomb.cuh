@@ -84,53 +84,100 @@ __device__ __forceinline__ cx<CT> up_to(cx<R> a) {
 
 // ---------------------------------------------------------------------
 // derivative on the rotated links W_i(x) = g(x) U_i(x) g(x+i)^dag, packed like
-// the Landau fields (steep_deriv_CG, src/Gfix/CFACG.c:91-163).  Only the
-// traceless anti-Hermitian part of sum_i W_i(x-i) - W_i(x) enters, and W and
-// -W^dag have the same one, so with
+// the Landau fields (steep_deriv_CG, src/Gfix/CFACG.c:91-163): the traceless
+// anti-Hermitian part of sum_i W_i(x-i) - W_i(x).
+//
+// In FP64 arithmetic the links are not formed.  W and -W^dag have the same
+// part, so with
 //   S(x) = sum_i U_i(x) g(x+i)^dag + (g(x-i) U_i(x-i))^dag
 // it is that of -g(x) S(x): one product for each of the six links and one
-// with g(x), in place of two for each.  At 32^3 x 64, FP64: 0.324 -> 0.215 ms
-// (0.74 of the copy bandwidth on its algorithmic bytes; four blocks per SM,
-// three take 0.228 ms), FP32 storage 0.236 -> 0.162 ms.
-template <typename R, typename CT, int MU>
-__device__ __forceinline__ void cderiv_dir(const CCtx<R> &c, const SliceSite &q,
-                                           int off, cx<CT> *S) {
-  const int it = sfwd<MU>(q, c.L), bk = sbck<MU>(q, c.L);
+// with g(x), in place of two for each.  Every column of a product is formed
+// from those of its factors: a third column completed from the first two would
+// differ, for a g off SU(3) (FP32 storage, or the drift of a long run), from
+// what the neighbour's sum holds of the same link, and the two would no longer
+// cancel in the sum over the slice, which turns the slice as a whole.  A
+// product's three terms are added before they meet the sum.  Rms error of a
+// site against 128 bits: 0.5 to 0.85 of that of six links formed by two products
+// each.  32^3 x 64: 0.326 -> 0.239 ms (four blocks per SM).
+//
+// FP32 arithmetic (FP32 storage, theta >= hp_below) forms the links: the same
+// bits at both ends of each, whose sum over the slice cancels to the last,
+// where the rounding of -g S in 32 bits turned the slice, and a mixed fix ended
+// 1.1 to 1.4 times as far from the same in 64 bits (0.16 instead of 0.23 ms).
+template <typename R, typename CT>
+__device__ __forceinline__ void link_ct(const CCtx<R> &c, int mu, int s, cx<CT> *U) {
   cx<R> t[9];
-  cx<CT> U[9], G[9];
-  load_link(c.U, c.V, MU, off + q.i, t);
+  load_link(c.U, c.V, mu, s, t);
 #pragma unroll
   for (int e = 0; e < 9; e++) U[e] = up_to<CT>(t[e]);
   if constexpr (sizeof(CT) != sizeof(R)) complete_col2(U);
-  load9(c.g, c.V, off + it, t);
+}
+template <typename R, typename CT>
+__device__ __forceinline__ void gauge_ct(const CCtx<R> &c, int s, cx<CT> *G) {
 #pragma unroll
-  for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t[e]);
+  for (int e = 0; e < 9; e++) G[e] = up_to<CT>(c.g[(size_t)e * c.V + s]);
+}
+// a b + s of row-times-column triples, the three terms first
+template <typename CT>
+__device__ __forceinline__ cx<CT> add_dot(cx<CT> s, cx<CT> a0, cx<CT> b0, cx<CT> a1, cx<CT> b1,
+                                          cx<CT> a2, cx<CT> b2) {
+  return cadd(s, cmadd(cmadd(cmul(a0, b0), a1, b1), a2, b2));
+}
+
+// S += U_MU(x) g(x+MU)^dag + (g(x-MU) U_MU(x-MU))^dag
+template <typename R, typename CT, int MU>
+__device__ __forceinline__ void cderiv_dir(const CCtx<R> &c, const SliceSite &q,
+                                           int off, cx<CT> *S) {
+  const int it = off + sfwd<MU>(q, c.L), bk = off + sbck<MU>(q, c.L);
+  cx<CT> U[9], G[9];
+  link_ct(c, MU, off + q.i, U);
+  gauge_ct(c, it, G);
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++)
+      S[3 * i + j] = add_dot(S[3 * i + j], U[3 * i], conjg(G[3 * j]), U[3 * i + 1],
+                             conjg(G[3 * j + 1]), U[3 * i + 2], conjg(G[3 * j + 2]));
+  link_ct(c, MU, bk, U);
+  gauge_ct(c, bk, G);
 #pragma unroll
-      for (int k = 0; k < 3; k++)
-        S[3 * i + j] = cmaddc(S[3 * i + j], U[3 * i + k], G[3 * j + k]);
-  // P = g(x-i) U(x-i): the first two columns, the third completed
-  cx<R> r0[3], r1[3];
-  cx<CT> u0[3], u1[3], p0[3], p1[3];
-  load_cols(c.U, c.V, MU, off + bk, r0, r1);
+  for (int k = 0; k < 3; k++)
 #pragma unroll
-  for (int r = 0; r < 3; r++) u0[r] = up_to<CT>(r0[r]), u1[r] = up_to<CT>(r1[r]);
-  load9(c.g, c.V, off + bk, t);
-#pragma unroll
-  for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t[e]);
-  mat_vec(p0, G, u0);
-  mat_vec(p1, G, u1);
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    S[r] = cadd(S[r], conjg(p0[r]));
-    S[3 + r] = cadd(S[3 + r], conjg(p1[r]));
-  }
-  S[6] = cadd(S[6], conjg(cdet(p0[1], p1[2], p0[2], p1[1])));
-  S[7] = cadd(S[7], conjg(cdet(p0[2], p1[0], p0[0], p1[2])));
-  S[8] = cadd(S[8], conjg(cdet(p0[0], p1[1], p0[1], p1[0])));
+    for (int r = 0; r < 3; r++)
+      S[3 * k + r] = add_dot(S[3 * k + r], conjg(G[3 * r]), conjg(U[k]), conjg(G[3 * r + 1]),
+                             conjg(U[3 + k]), conjg(G[3 * r + 2]), conjg(U[6 + k]));
+}
+
+// Hermitian short form of a matrix (herm_short)
+template <typename CT>
+struct HShort {
+  CT h0, h3;
+  cx<CT> h1, h2, h4;
+};
+// that of the link g(a) U_MU(a) g(b)^dag
+template <typename R, typename CT>
+__device__ __forceinline__ HShort<CT> rotated_herm(const CCtx<R> &c, int mu, int a, int b) {
+  cx<CT> C[9], A[9], B[9];
+  link_ct(c, mu, a, C);
+  gauge_ct(c, a, A);
+  gauge_ct(c, b, B);
+  gtransform(A, C, B);
+  HShort<CT> h;
+  herm_short(C, h.h0, h.h1, h.h2, h.h3, h.h4);
+  return h;
+}
+// H += that of W_MU(x-MU), less that of W_MU(x)
+template <typename R, typename CT, int MU>
+__device__ __forceinline__ void cderiv_links(const CCtx<R> &c, const SliceSite &q, int off,
+                                             HShort<CT> &H) {
+  const int x = off + q.i, it = off + sfwd<MU>(q, c.L), bk = off + sbck<MU>(q, c.L);
+  const HShort<CT> b = rotated_herm<R, CT>(c, MU, x, it);
+  const HShort<CT> a = rotated_herm<R, CT>(c, MU, bk, x);
+  H.h0 += a.h0 - b.h0;
+  H.h1 = cadd(H.h1, csub(a.h1, b.h1));
+  H.h2 = cadd(H.h2, csub(a.h2, b.h2));
+  H.h3 += a.h3 - b.h3;
+  H.h4 = cadd(H.h4, csub(a.h4, b.h4));
 }
 
 // CT: arithmetic type.  With FP32 storage a slice below theta = hp_below is
@@ -146,35 +193,38 @@ __global__ void __launch_bounds__(kCoulThreads, 4) k_cderiv(CCtx<R> c, int sel) 
   if (i >= c.Lcu) return;
   const SliceSite q = slice_site(i, c.L);
   const int off = t * c.Lcu;
-  cx<CT> S[9], G[9], M[9];
+  HShort<CT> H;  // the sum's Hermitian short form
+  if constexpr (sizeof(CT) == 4) {
+    H.h0 = H.h3 = 0;
+    H.h1 = H.h2 = H.h4 = mk<CT>(0, 0);
+    cderiv_links<R, CT, 0>(c, q, off, H);
+    cderiv_links<R, CT, 1>(c, q, off, H);
+    cderiv_links<R, CT, 2>(c, q, off, H);
+  } else {
+    cx<CT> S[9], G[9], M[9];
 #pragma unroll
-  for (int e = 0; e < 9; e++) S[e] = mk<CT>(0, 0);
-  cderiv_dir<R, CT, 0>(c, q, off, S);
-  cderiv_dir<R, CT, 1>(c, q, off, S);
-  cderiv_dir<R, CT, 2>(c, q, off, S);
-  {
-    cx<R> t9[9];
-    load9(c.g, c.V, off + i, t9);
+    for (int e = 0; e < 9; e++) S[e] = mk<CT>(0, 0);
+    cderiv_dir<R, CT, 0>(c, q, off, S);
+    cderiv_dir<R, CT, 1>(c, q, off, S);
+    cderiv_dir<R, CT, 2>(c, q, off, S);
+    gauge_ct(c, off + i, G);
 #pragma unroll
-    for (int e = 0; e < 9; e++) G[e] = up_to<CT>(t9[e]);
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const cx<CT> m = cmadd(cmadd(cmul(G[3 * r], S[k]), G[3 * r + 1], S[3 + k]),
+                               G[3 * r + 2], S[6 + k]);
+        M[3 * r + k] = mk<CT>(-m.x, -m.y);
+      }
+    herm_short(M, H.h0, H.h1, H.h2, H.h3, H.h4);
   }
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-      M[3 * r + k] = cmadd(cmadd(cmul(G[3 * r], S[k]), G[3 * r + 1], S[3 + k]),
-                           G[3 * r + 2], S[6 + k]);
-  CT s0, s3;
-  cx<CT> s1, s2, s4;
-  herm_short(M, s0, s1, s2, s3, s4);
-  // pack: in0 = i Re s0 - Re s3, in_k = i Re s_k - Im s_k of -g S
-  // (CFACG.c:144-150)
+  // pack: in0 = i Re s0 - Re s3, in_k = i Re s_k - Im s_k (CFACG.c:144-150)
   cx<R> *f = pick(c.fb, c.st->parity);
   const size_t V = c.V, s = off + i;
-  f[s] = mk<R>((R)s3, (R)-s0);
-  f[V + s] = mk<R>((R)s1.y, (R)-s1.x);
-  f[2 * V + s] = mk<R>((R)s2.y, (R)-s2.x);
-  f[3 * V + s] = mk<R>((R)s4.y, (R)-s4.x);
+  f[s] = mk<R>((R)-H.h3, (R)H.h0);
+  f[V + s] = mk<R>((R)-H.h1.y, (R)H.h1.x);
+  f[2 * V + s] = mk<R>((R)-H.h2.y, (R)H.h2.x);
+  f[3 * V + s] = mk<R>((R)-H.h4.y, (R)H.h4.x);
 }
 
 // The sums of the accelerated field, insum (sum_DER2 / sum_PR, one norm) and

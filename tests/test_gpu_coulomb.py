@@ -268,3 +268,35 @@ def test_slice_blocks_equal_whole_lattice(lat400, blocks):
     got = np.concatenate([b.cpu().numpy() for b, _ in dev]).view(np.complex128)
     assert np.array_equal(got.reshape(whole.links.shape), whole.links)
     assert np.array_equal(np.concatenate(its), whole.slice_iters)
+
+
+def _su3(c0, c1):
+    c0 = c0 / np.linalg.norm(c0, axis=-1, keepdims=True)
+    c1 = c1 - np.sum(np.conj(c0) * c1, axis=-1, keepdims=True) * c0
+    c1 = c1 / np.linalg.norm(c1, axis=-1, keepdims=True)
+    return np.stack([c0, c1, np.conj(np.cross(c0, c1))], axis=-1)
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_fp32_storage_leaves_the_slices_where_they_are(hb8, seed):
+    """The sum of the derivative over a slice is zero, whatever g: what each
+    site holds of a link cancels what its neighbour does.  On smooth links near
+    their gauge (theta below 1e-2, FP64 arithmetic on g rounded to FP32), a sum
+    that does not cancel turns the slices against the FP64 fix."""
+    dims = _dims(hb8)
+    rng = np.random.default_rng(seed)
+    V = int(np.prod(dims))
+    u, one = hb8["links"].reshape(V, 4, 3, 3), np.eye(3)
+    u = _su3(u[..., 0] + 2 * one[0], u[..., 1] + 2 * one[1])
+    z = rng.normal(size=(2, V, 3)) + 1j * rng.normal(size=(2, V, 3))
+    G = _su3(50 * one[0] + z[0], 50 * one[1] + z[1])
+    idx = np.arange(V).reshape(dims[::-1])
+    for mu in range(4):
+        fwd = np.roll(idx, -1, axis=3 - mu).reshape(V)
+        u[:, mu] = G @ u[:, mu] @ np.conj(np.swapaxes(G[fwd], -1, -2))
+    a = gfix.coulomb_fix(u, dims, 0.08, ACC, 2000, "FACG").links
+    b = gfix.coulomb_fix(u, dims, 0.08, ACC, 2000, "FACG", precision="MIXED").links
+    # what the rounding of the fields to FP32 leaves: their sum over the 512
+    # sites of a slice, 3e-8 of a derivative of 1e-2 at each
+    d = np.linalg.norm(a - b) / np.linalg.norm(a)
+    assert d < 9e-9, d
