@@ -378,6 +378,15 @@ static __global__ void __launch_bounds__(kScalarThreads)
 // the iteration, which flips sn's buffers, has been applied with the probes').
 // With G (mixed precision) the transform is accumulated, G(x) <- g(x) G(x).
 //
+// A link's third column is completed from its first two (as GLU does), so a
+// departure from SU(3) passes on multiplied: by up to 4/3 for gauge rotations
+// of order one, less on a plateau.  Left alone it reaches 5e-8 after 900
+// iterations at 32^3 x 64 and takes a fix of 48^3 x 96 off its gauge orbit
+// (plaquette 6e-8 off); so FP64 links are reunitarised every kReunitEvery
+// iterations, in which a departure grows tenfold at most.  (FP32 links are not:
+// the phase they serve ends on the FP64 input's orbit in any case, and took
+// more iterations with it.)
+//
 // Bound by the bytes of links and fields.  In FP64 the registers allow three
 // blocks per SM, whose loads alone don't cover the latency between two
 // directions: each thread fetches the next direction's link and neighbour to
@@ -385,6 +394,8 @@ static __global__ void __launch_bounds__(kScalarThreads)
 // (0.93 of the copy bandwidth; FP32 fields 0.321 -> 0.285), 48^3 x 96 1.676 ->
 // 1.418 (0.95), 24^3 x 48 0.110 -> 0.095.  FP32 links are at 0.94 to 0.97 as
 // they are.
+
+constexpr int kReunitEvery = 8;
 
 template <typename R, bool SN, typename F = R>
 __global__ void __launch_bounds__(kSiteThreads) k_update(Ctx<R, F> c) {
@@ -405,6 +416,7 @@ __global__ void __launch_bounds__(kSiteThreads) k_update(Ctx<R, F> c) {
     __shared__ cx<R> sU[kLinkCx][kSiteThreads];
     __shared__ cx<F> sF[4][kSiteThreads];
     const int tid = threadIdx.x;
+    const bool reunit = c.st->iter % kReunitEvery == kReunitEvery - 1;
     auto fetch = [&](int mu) {
       const int y = fwd_site(s, mu, x, c.L, sd);
 #pragma unroll
@@ -428,6 +440,7 @@ __global__ void __launch_bounds__(kSiteThreads) k_update(Ctx<R, F> c) {
       complete_col2(U);
       set_gauge(Bm, up(f[0]), up(f[1]), up(f[2]), up(f[3]), alpha);
       gtransform(A, U, Bm);
+      if (reunit) gram_reunit(U);
       store_link(c.U, c.V, mu, s, U);
     }
   } else {

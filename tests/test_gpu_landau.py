@@ -11,6 +11,7 @@ if not torch.cuda.is_available():
     pytest.skip("no CUDA device", allow_module_level=True)
 
 from glu_b200 import gfix  # noqa: E402
+from glu_b200.workload import random_su3  # noqa: E402
 
 
 def _rel(a, b):
@@ -249,3 +250,19 @@ def test_gf_check_matches_reference(reference, case, which, request):
         assert abs(got[k] - r) <= tol * abs(r) + floor, (k, got[k], r)
     text = gfix.gf_check_report(got)
     assert "[GFACC LANDAU]      LOG ::" in text and "[GFACC MAX COULOMB] LOG ::" in text
+
+
+@pytest.mark.parametrize("algo, alpha", [("FASD", 0.6), ("FASD", 0.3)])
+def test_links_stay_on_their_orbit_over_a_long_run(algo, alpha):
+    """Steps too long to converge, each a gauge rotation of order one, over
+    which a departure from SU(3) grows by a fifth an iteration where nothing
+    takes it back (3e-2 after 200; the plaquette 7e-6 off)."""
+    dims = (4, 4, 4, 8)
+    V = int(np.prod(dims))
+    U = random_su3(4 * V, np.random.default_rng(3)).reshape(V, 4, 3, 3)
+    r = gfix.landau_fix(U, dims, alpha, 1e-30, 200, algo, sd_fixed_step=True)
+    assert np.abs(r.links - U).max() > 0.1
+    # rounding of some 20 products and eight iterations' growth, 4/3 each
+    dep = np.abs(r.links @ np.conj(np.swapaxes(r.links, -1, -2)) - np.eye(3)).max()
+    assert dep < 20 * 1.2e-16 * 10 * 8
+    assert abs(gfix.av_plaquette(r.links, dims) - gfix.av_plaquette(U, dims)) < 1e-13
