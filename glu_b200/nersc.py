@@ -25,14 +25,6 @@ _FP = {"IEEE64BIG": (8, True), "IEEE32BIG": (4, True), "IEEE32": (4, True),
 _TYPES = {"4D_SU3_GAUGE": 12, "4D_SU3_GAUGE_3x3": 18}
 
 
-# a bytes object of n bytes not yet written, for a call to fill before anyone
-# else holds it: a copy of the payload (50 to 75 MB at 16^3 x 32) less
-_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.restype, _new_bytes.argtypes = C.py_object, (C.c_char_p, C.c_ssize_t)
-_bytes_at = C.pythonapi.PyBytes_AsString
-_bytes_at.restype, _bytes_at.argtypes = C.c_void_p, (C.py_object,)
-
-
 class NerscError(RuntimeError):
     pass
 
@@ -76,14 +68,14 @@ def encode(links, dims, nreal=12, bytes_per_real=8, big_endian=True):
     lib = _lib.load()
     d = tuple(int(x) for x in dims)
     U = np.ascontiguousarray(links, dtype=np.complex128).reshape(-1, 4, 3, 3)
-    out = _new_bytes(None, max(U.shape[0] * 4 * nreal * bytes_per_real, 0))
+    out = np.empty(U.shape[0] * 4 * nreal * bytes_per_real, dtype=np.uint8)
     ck = C.c_uint32(0)
     rc = lib.gfix_nersc_encode(U.ctypes.data, (C.c_size_t * 4)(*d), nreal,
-                               bytes_per_real, int(big_endian), _bytes_at(out),
+                               bytes_per_real, int(big_endian), out.ctypes.data,
                                C.byref(ck))
     if rc != 0:
         raise NerscError(lib.gfix_nersc_error().decode())
-    return out, int(ck.value)
+    return out.tobytes(), int(ck.value)
 
 
 def read(path, check=True):
