@@ -47,3 +47,12 @@ def test_ildg_records_and_scidac_checksum_of_the_fixture_file():
             else:
                 b ^= v
     assert (a, b) == (suma, sumb)
+
+
+def test_the_interpreters_own_functions_keep_their_prototypes():
+    """ctypes.pythonapi's functions are shared by the whole process."""
+    import ctypes as C
+
+    import glu_b200.nersc  # noqa: F401
+    assert C.pythonapi.PyBytes_AsString.restype is C.c_int
+    assert C.pythonapi.PyBytes_FromStringAndSize.argtypes is None
