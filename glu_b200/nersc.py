@@ -68,6 +68,8 @@ def encode(links, dims, nreal=12, bytes_per_real=8, big_endian=True):
     lib = _lib.load()
     d = tuple(int(x) for x in dims)
     U = np.ascontiguousarray(links, dtype=np.complex128).reshape(-1, 4, 3, 3)
+    if U.shape[0] != int(np.prod(d)):
+        raise NerscError(f"links hold {U.shape[0]} sites, dims {d} need {int(np.prod(d))}")
     out = np.empty(U.shape[0] * 4 * nreal * bytes_per_real, dtype=np.uint8)
     ck = C.c_uint32(0)
     rc = lib.gfix_nersc_encode(U.ctypes.data, (C.c_size_t * 4)(*d), nreal,

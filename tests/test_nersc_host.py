@@ -3,8 +3,9 @@
 from pathlib import Path
 
 import numpy as np
+import pytest
 
-from glu_b200.nersc import parse_header
+from glu_b200.nersc import NerscError, encode, parse_header
 
 FILE = Path(__file__).resolve().parent / "golden" / "lat400.nersc"
 
@@ -56,3 +57,10 @@ def test_the_interpreters_own_functions_keep_their_prototypes():
     import glu_b200.nersc  # noqa: F401
     assert C.pythonapi.PyBytes_AsString.restype is C.c_int
     assert C.pythonapi.PyBytes_FromStringAndSize.argtypes is None
+
+
+@pytest.mark.parametrize("sites", [0, 7, 9, 32])
+def test_encode_refuses_links_of_another_lattice(sites):
+    """The codec reads and writes as many sites as the extents say."""
+    with pytest.raises(NerscError, match="sites"):
+        encode(np.zeros((sites, 4, 3, 3), dtype=np.complex128), (2, 2, 2, 1))
