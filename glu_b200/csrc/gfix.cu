@@ -542,16 +542,18 @@ class Engine {
   }
 
   // --- launch sequences ------------------------------------------------
-  // the blocks of a kernel over the sites: as many as the SMs hold at once
+  // the blocks of a kernel over the sites: as many as the SMs of a B200 hold at
+  // once.  Not the SMs of this device, fewer on a share of one: the order of the
+  // sums, and with it an iteration count, is a matter of the lattice alone (no
+  // block waits for another).
+  static constexpr int kSms = 148;
   template <typename K>
   int fill(K k, bool whole = false) {
     int &n = resident[(const void *)k];
     if (n == 0) {
-      int per = 0, dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      int per = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kSiteThreads, 0);
-      n = std::max(1, per * sms);
+      n = std::max(1, per * kSms);
     }
     return whole ? n : std::min(n, nb_site);
   }
