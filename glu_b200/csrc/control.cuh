@@ -19,7 +19,6 @@
 
 namespace gfix {
 
-constexpr double kCgTol = 5E-11;            // GLU_definitions.h:451-455
 constexpr double kVal49 = 0.4444444444444444;  // lin_derivs.c:72
 constexpr int kSiteThreads = 128;
 

@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(kCoulThreads, sizeof(CT) == 4 ? 4 : 3) k_cprob
 // src/Gfix/line_search.c:101-115)
 template <typename R>
 __global__ void __launch_bounds__(kCoulThreads) k_cupdate(CCtx<R> c) {
-  // (from the last site to the first, as k_update)
+  // (from the last site to the first, whose g and fields the probes before it
+  // left in L2: 32^3 x 64 0.126 -> 0.123 ms in FP64, 0.0585 -> 0.0556 in FP32)
   const int t = gridDim.y - 1 - blockIdx.y;
   const Slice &S = c.sl[t];
   if (S.mode == SL_DONE) return;

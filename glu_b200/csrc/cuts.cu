@@ -17,9 +17,9 @@
 //                 writes the packed fields first
 //   k_cut_zt      z and t transforms of tiles of x columns
 //                 (both also as k_cut_*_ct with compile-time extents)
-//   k_cut_pxy, k_cut_pz, k_cut_pt  instead of the full transforms, where the
-//                 cut keeps few momenta of each axis: every axis is summed
-//                 into its kept components alone
+//   k_cut_pxy, k_cut_part  instead of the full transforms, where the cut keeps
+//                 few momenta of each axis: x and y, then z, then t are summed
+//                 into their kept components alone
 //   k_cut_gather  per listed momentum: A_mu(p) for all 9 colour entries
 //                 from the packed transforms at p and -p (the transform of
 //                 a real field R obeys R(-p) = conj R(p), and of conj(f)

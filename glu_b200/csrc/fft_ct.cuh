@@ -1,66 +1,13 @@
-// Compile-time specialised FFT passes for the usual extents whose register
-// pencils (fft_reg.cuh) would need more registers than a thread has (FP64: 48
-// and 64, Coulomb z pencils of 32; FP32: Coulomb z pencils of 64).  Same
-// algorithm, tiles and results as the
-// generic passes in fft_pass.cuh (in-place Stockham stages in shared memory,
-// radix 8/4/2/3, twiddles staged in shared memory), but every extent, stride
-// and pencil mapping is a template constant, so the per-butterfly index
-// arithmetic folds to shifts and multiply-adds and every loop unrolls.
+// Compile-time specialised z(,t) passes for the usual extents whose register
+// pencils (fft_reg.cuh) would need more registers than a thread has (FP64: 48 x
+// 96 one column wide, Coulomb z pencils of 32 and 48; Coulomb z pencils of 64).
+// Same algorithm, tiles and results as the generic passes in fft_pass.cuh
+// (in-place Stockham stages in shared memory, radix 8/4/2/3, twiddles staged in
+// shared memory), but every extent, stride and pencil mapping is a template
+// constant, so the per-butterfly index arithmetic folds to shifts and
+// multiply-adds and every loop unrolls.
 // Included by kernels.cuh inside namespace gfix, after fft_pass.cuh; the
 // stage template ct_stages is in fft.cuh.
-
-// xy-plane pass with compile-time extents (see k_fft_xy)
-template <typename R, int LX, int LY>
-__global__ void __launch_bounds__(ct_threads(LX *LY), ct_minb(LX *LY))
-    k_fft_xy_ct(Ctx<R> c, int bwd, int prsum) {
-  if (xy_done(c, bwd)) return;
-  if (c.skip && c.skip[blockIdx.x / c.L[2]]) return;  // finished slice
-  constexpr int P = LX + 1, N = LX * LY, BD = ct_threads(N);
-  constexpr int EPT = (N + BD - 1) / BD;
-  extern __shared__ unsigned char smem_raw[];
-  cx<R> *A = reinterpret_cast<cx<R> *>(smem_raw);
-  cx<R> *twx = A + P * LY;
-  cx<R> *twy = twx + LX;
-  stage_twiddles(twx, c.tw + c.ax[0].tw_off, LX);
-  stage_twiddles(twy, c.tw + c.ax[1].tw_off, LY);
-  const int plane = blockIdx.x, field = blockIdx.y;
-  const int par = c.st->parity;
-  const size_t base = (size_t)field * c.V + (size_t)plane * N;
-  cx<R> *data = c.fb[par] + base;
-#pragma unroll
-  for (int k = 0; k < EPT; k++) {
-    const int e = threadIdx.x + k * BD;
-    if (N % BD == 0 || e < N) A[(e / LX) * P + e % LX] = data[e];
-  }
-  __syncthreads();
-  ct_stages<R, LX, 1, LY, 1, 0, P, 1, BD>(A, twx, bwd != 0);   // rows
-  ct_stages<R, LY, 1, LX, LX, 1, 0, P, BD>(A, twy, bwd != 0);  // columns
-  double v[2] = {0.0, 0.0};
-  const cx<R> *old = c.fb[par ^ 1] + base;
-#pragma unroll
-  for (int k = 0; k < EPT; k++) {
-    const int e = threadIdx.x + k * BD;
-    if (N % BD != 0 && e >= N) continue;
-    const cx<R> w = A[(e / LX) * P + e % LX];
-    data[e] = w;
-    if (prsum) {
-      const cx<R> od = old[e];
-      const double a = w.x, b = w.y;
-      const double tr = a - (double)od.x, ti = b - (double)od.y;
-      if (field == 0) {
-        v[0] += 2.0 * (a * a + b * b + a * b);
-        v[1] += 2.0 * (a * tr + b * ti) + (a * ti + b * tr);
-      } else {
-        v[0] += 2.0 * (a * a + b * b);
-        v[1] += 2.0 * (a * tr + b * ti);
-      }
-    }
-  }
-  if (prsum) {
-    xy_sums_begin<BD % 32 != 0>(c, v);
-    xy_sums<BD % 32 != 0>(c, v);
-  }
-}
 
 // z(,t) pass with compile-time extents (see k_fft_zt).  NT = Lt for Landau
 // (z and t transformed); NT = 1 for Coulomb (z only, one slice per tile).

@@ -80,31 +80,21 @@ static int fft_tuning() {
   return g_fft_tune;
 }
 
-// compile-time specialised FFT passes for the common extents; nullptr
-// where the generic passes serve
 template <typename R>
 using XyFn = void (*)(Ctx<R>, int, int);
 template <typename R>
 using ZtFn = void (*)(Ctx<R>);
 
-// (the extents whose register-pencil passes would need more registers than a
-// thread has: fft_reg_api.cuh)
-template <typename R>
-static XyFn<R> ct_xy(int lx, int ly) {
-  if constexpr (sizeof(R) == 8) {
-    if (lx == 48 && ly == 48) return k_fft_xy_ct<R, 48, 48>;
-    if (lx == 64 && ly == 64) return k_fft_xy_ct<R, 64, 64>;
-  }
-  return nullptr;
-}
-
+// compile-time z(,t) passes of usual extents whose register pencils
+// (fft_reg_api.cuh) would need more registers than a thread has; nullptr where
+// those or the generic passes serve
 template <typename R>
 static ZtFn<R> ct_zt(int lz, int lt, int b) {
 #define GFIX_ZT(z, t, bb) \
   if (lz == z && lt == t && b == bb) return k_fft_zt_ct<R, z, t, bb>;
   GFIX_ZT(64, 1, 8) GFIX_ZT(64, 1, 16) GFIX_ZT(64, 1, 32)
   if constexpr (sizeof(R) == 8) {
-    GFIX_ZT(48, 96, 2) GFIX_ZT(48, 96, 1) GFIX_ZT(48, 1, 8) GFIX_ZT(48, 1, 16)
+    GFIX_ZT(48, 96, 1) GFIX_ZT(48, 1, 8) GFIX_ZT(48, 1, 16)
     GFIX_ZT(32, 1, 8) GFIX_ZT(32, 1, 16) GFIX_ZT(32, 1, 32)
   }
 #undef GFIX_ZT
@@ -380,9 +370,8 @@ class Engine {
                             (int)cudaSharedmemCarveoutMaxShared));
     return 0;
   }
-  // the xy pass: compile-time (use_ct; register pencils, or the staged form
-  // where those do not reach) or generic with radix order `order`; -1 where
-  // that pass does not exist for these extents
+  // the xy pass: compile-time (use_ct; register pencils) or generic with radix
+  // order `order`; -1 where that pass does not exist for these extents
   int apply_xy(bool use_ct, int order) {
     for (int a = 0; a < 2; a++)
       if (factorize(c.L[a], c.ax[a], order)) return -1;
@@ -393,22 +382,14 @@ class Engine {
     if (use_ct) {
       const RegXy<F> r = c.L[0] == c.L[1] ? reg_xy<F>(c.L[0], coul ? c.L[2] : c.L[2] * c.L[3])
                                           : RegXy<F>{};
-      XyFn<F> fn = odd ? nullptr : ct_xy<F>(c.L[0], c.L[1]);
-      if (r.fn[0]) {
-        for (int k = 0; k < 2; k++) {
-          xy_ct[k] = r.fn[k];
-          if (shared_limit(r.fn[k], r.smem)) return -1;
-        }
-        bd_xy = r.threads;
-        sm_xy = r.smem;
-        planes = r.planes;
-      } else if (fn) {
-        xy_ct[0] = xy_ct[1] = fn;
-        bd_xy = ct_threads((int)n);
-        if (shared_limit(fn, sm_xy)) return -1;
-      } else {
-        return -1;
+      if (!r.fn[0]) return -1;
+      for (int k = 0; k < 2; k++) {
+        xy_ct[k] = r.fn[k];
+        if (shared_limit(r.fn[k], r.smem)) return -1;
       }
+      bd_xy = r.threads;
+      sm_xy = r.smem;
+      planes = r.planes;
     } else {
       xy_ct[0] = xy_ct[1] = nullptr;
       pt_xy = (n <= 4096u && !odd) ? 8 : 16;

@@ -10,8 +10,8 @@
 //                      only columns 0 and 1 filled (src/Gfix/CG.c:72-97)
 //   gtransform         b <- a b c^dag, columns 0,1 explicit, column 2 by
 //                      conj cross product (src/Gfix/gtrans.c:31-141)
-//   re_tr_abc_dag      Re tr(a b c^dag), row 2 of ab by cross product
-//                      (src/Matrix_Ops/trace_abc_SSE.c:34-114)
+//   probe_trace        Re tr(a b c^dag) (src/Matrix_Ops/trace_abc_SSE.c:34-114)
+//                      of the line search, c = reunit(1 + alpha A) not formed
 //   multab             a <- b c, row 2 by cross product
 //                      (src/Matrix_Ops/MMUL/MMUL_SUNC_SSE.c:30-76)
 #pragma once
@@ -155,34 +155,6 @@ __device__ __forceinline__ void gtransform(const cx<R> *a, cx<R> *b,
     }
   }
   complete_col2(b);
-}
-
-// Re tr(a b c^dag), row 2 of (a b) completed by the cross product
-template <typename R>
-__device__ __forceinline__ R re_tr_abc_dag(const cx<R> *a, const cx<R> *b,
-                                           const cx<R> *c) {
-  cx<R> ab[9];
-#pragma unroll
-  for (int r = 0; r < 2; r++) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      ab[r * 3 + k] = cadd(cadd(cmul(a[r * 3 + 0], b[k]),
-                                cmul(a[r * 3 + 1], b[3 + k])),
-                           cmul(a[r * 3 + 2], b[6 + k]));
-    }
-  }
-  ab[6] = conjg(csub(cmul(ab[1], ab[5]), cmul(ab[2], ab[4])));
-  ab[7] = conjg(csub(cmul(ab[2], ab[3]), cmul(ab[0], ab[5])));
-  ab[8] = conjg(csub(cmul(ab[0], ab[4]), cmul(ab[1], ab[3])));
-  R sr = R(0), si = R(0);
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    sr += (ab[r * 3 + 2].x * c[r * 3 + 2].x + ab[r * 3 + 1].x * c[r * 3 + 1].x) +
-          ab[r * 3 + 0].x * c[r * 3 + 0].x;
-    si += (ab[r * 3 + 2].y * c[r * 3 + 2].y + ab[r * 3 + 1].y * c[r * 3 + 1].y) +
-          ab[r * 3 + 0].y * c[r * 3 + 0].y;
-  }
-  return sr + si;
 }
 
 // acc + a b, four fused operations
