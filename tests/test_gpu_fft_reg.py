@@ -76,3 +76,54 @@ def test_fp32_passes_follow_fp64(dims):
     # and the transforms multiply that by their log2 V stages
     assert np.abs(m - w).max() < 2e-5
     assert np.linalg.norm(m - w) < 2e-6 * np.linalg.norm(w)
+
+
+def _links(dims, seed):
+    from glu_b200.workload import random_su3
+    V = int(np.prod(dims))
+    return random_su3(4 * V, np.random.default_rng(seed)).reshape(V, 4, 3, 3)
+
+
+# planes of every compiled width, in runs of four, two and one to a block, and
+# blocks whose last warp is not whole
+PLANES = [(n, n, z, t) for n in (4, 6, 10, 14, 18, 20, 28, 30, 32, 36, 40, 48, 64)
+          for z, t in ((2, 2), (3, 2), (3, 3))]
+
+
+@pytest.mark.parametrize("dims", PLANES)
+def test_conjugate_gradient_sums(oracle, dims):
+    """Three iterations of conjugate gradients: beta comes from the sums that
+    the inverse xy passes take of the new and the previous fields, theta and the
+    links after them show it."""
+    U = _links(dims, 5)
+    w = oracle.landau(U, dims, 0.08, 1e-30, 3, "FACG", traj_cap=8)
+    r = gfix.landau_fix(U, dims, 0.08, 1e-30, 3, "FACG", traj_cap=8)
+    n = len(w["traj_theta"])
+    assert n >= 4
+    # rounding of the sums and transforms, through four line searches
+    assert np.abs(r.traj_theta[:n] / w["traj_theta"] - 1).max() < 1e-11
+    assert np.abs(r.links.ravel() - np.asarray(w["links"]).ravel()).max() < 1e-9
+    m = gfix.landau_fix(U, dims, 0.08, 1e-30, 3, "FACG", precision="MIXED", traj_cap=8)
+    # the same in FP32: 6e-8 of the fields in each of the four
+    assert np.abs(m.traj_theta[:n] / w["traj_theta"] - 1).max() < 1e-4
+
+
+@pytest.mark.parametrize("dims", [(n, n, n, 2) for n in (6, 10, 14, 18, 20, 28, 30, 36, 40, 48)]
+                         + [(64, 64, 4, 2), (36, 36, 5, 3), (40, 40, 10, 2), (10, 10, 30, 3)])
+def test_coulomb_sums_and_fp32_passes(dims):
+    """Smooth slices come to theta < 1e-6 in as many steps by the FP32 passes
+    and sums as by the FP64 ones, whose z passes are others (fft_reg.cuh,
+    fft_ct.cuh or generic by the extent)."""
+    rng = np.random.default_rng(6)
+    V = int(np.prod(dims))
+    z = 4 * np.eye(3)[:, :2] + rng.normal(size=(V, 4, 3, 2)) + 1j * rng.normal(size=(V, 4, 3, 2))
+    c0 = z[..., 0] / np.linalg.norm(z[..., 0], axis=-1, keepdims=True)
+    c1 = z[..., 1] - np.sum(np.conj(c0) * z[..., 1], axis=-1, keepdims=True) * c0
+    c1 /= np.linalg.norm(c1, axis=-1, keepdims=True)
+    U = np.stack([c0, c1, np.conj(np.cross(c0, c1))], axis=-1)
+    a = gfix.coulomb_fix(U, dims, 0.08, 1e-6, 200, "FACG")
+    b = gfix.coulomb_fix(U, dims, 0.08, 1e-6, 200, "FACG", precision="MIXED", switch_theta=1e-6)
+    assert np.all(a.slice_theta < 1e-6) and np.all(b.slice_theta < 1e-6)
+    assert 3 * dims[3] < a.iters < 60 * dims[3]
+    # rounding moves a theta near the mark past it: a step for each slice
+    assert abs(b.iters_fp32 - a.iters) <= dims[3]
